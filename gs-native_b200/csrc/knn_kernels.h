@@ -8,8 +8,7 @@ namespace gsn {
 
 // Byte offsets of the sub-buffers of the KNN workspace for n points.
 struct KnnLayout {
-    int leaves;
-    size_t bounds, keys, keys_alt, ids, ids_alt, lo, hi, status, sort, total;
+    size_t bounds, keys, keys_alt, ids, ids_alt, sorted, lo, hi, sort, total;
 };
 KnnLayout knn_layout(int n);
 

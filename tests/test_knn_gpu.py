@@ -73,6 +73,24 @@ def test_neighbor_indices_equal_exhaustive_fp32_search():
     assert np.allclose(mean, expected, rtol=1e-6, atol=0)
 
 
+@pytest.mark.parametrize("n", [31, 33, 255, 257, 8191, 8193, 12001])
+def test_neighbors_at_the_edges_of_warps_and_tree_levels(n):
+    # a level of 32-child boxes is added past 256 and past 8,192 points; clusters,
+    # a far outlier and non-finite points, which have and are no neighbours
+    rng = np.random.default_rng(n)
+    pts = (rng.normal(0, 1, (n, 3)) + 20.0 * rng.integers(0, 3, (n, 1))).astype(np.float32)
+    pts[n // 2] = 1e6
+    finite = np.ones(n, bool)
+    if n > 1000:
+        pts[7, 1], pts[n - 2, 0] = np.nan, np.inf
+        finite[[7, n - 2]] = False
+    mean, nb = gsn.knn3_host(pts, neighbors=True)
+    keep = np.flatnonzero(finite)
+    _, idx = fp32_exhaustive(pts[keep])
+    assert np.array_equal(nb[keep], keep[idx])
+    assert np.all(np.isinf(mean[~finite])) and np.all(nb[~finite] == -1)
+
+
 def test_matches_reference_cuda_implementation():
     if not oracle.ref_available():
         pytest.skip("reference CUDA build not available")
