@@ -17,6 +17,9 @@ int launch_mlp_infer(const float* features, int n, const void* weights_f16, floa
 // and, when loss is given, adds that loss to *loss (FP64).
 int launch_mlp_gradients(const float* features, const int* labels, const float* sample_weights, int n,
                          float weight_norm, const void* weights_f16, float* grad, double* loss, cudaStream_t stream);
+// sums[0..kMlpWeightSums) (device): FP64 sums whose total is the sum of weights[0..n).
+constexpr int kMlpWeightSums = 128;
+int launch_mlp_weight_sum(const float* weights, int n, double* sums, cudaStream_t stream);
 // Adam step of the fp32 master weights (lr, bias corrections c1, c2); writes the
 // fp16 copy and clears grad.
 int launch_mlp_adam(float* master, float* m, float* v, float* grad, void* weights_f16, float lr, float c1, float c2,

@@ -50,12 +50,14 @@ bool DensityMlp::GetWeights(float* host) const {
 }
 
 double DensityMlp::WeightSum(const float* weights, int n) {
-    std::vector<float> w(static_cast<size_t>(n));
-    if (cudaMemcpyAsync(w.data(), weights, w.size() * sizeof(float), cudaMemcpyDeviceToHost, stream_) != cudaSuccess ||
+    double w[gsn::kMlpWeightSums];
+    if (!weight_sums_.Reserve(gsn::kMlpWeightSums) ||
+        gsn::launch_mlp_weight_sum(weights, n, weight_sums_.get(), stream_) != GSN_OK ||
+        cudaMemcpyAsync(w, weight_sums_.get(), sizeof(w), cudaMemcpyDeviceToHost, stream_) != cudaSuccess ||
         cudaStreamSynchronize(stream_) != cudaSuccess)
         return -1.0;
     double s = 0.0;
-    for (float x : w) s += x;
+    for (double x : w) s += x;
     return s;
 }
 

@@ -43,7 +43,7 @@ private:
     cudaStream_t stream_ = nullptr;
     DeviceArray<float> master_, m_, v_, grad_;
     DeviceArray<uint16_t> half_;
-    DeviceArray<double> loss_;
+    DeviceArray<double> loss_, weight_sums_;
     uint64_t step_ = 0;
 };
 

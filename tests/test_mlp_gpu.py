@@ -43,6 +43,33 @@ def test_gpu_gradients_match_fp64_oracle():
     assert np.max(np.abs(g - gref)) <= 1e-4 * np.max(np.abs(gref)) + 1e-7
 
 
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 2000, 40001])
+def test_ragged_tiles_match_the_fp64_oracle(n):
+    """Sizes around the 64-sample tile, one tile, fewer tiles than CTAs and several
+    per CTA: gradients as above, probabilities and confident actions of the inference."""
+    f, labels, w = samples(n, n)
+    mlp = gsn.Mlp(seed=n)
+    w16 = mlp.weights().astype(np.float16).astype(np.float64)
+    fd, ld, wd = dev(f), dev(labels), dev(w)
+    g, loss = mlp.gradients(fd.data_ptr(), ld.data_ptr(), wd.data_ptr(), n)
+    lref, gref = oracle.mlp_loss_gradient(w16, f, labels, w)
+    assert abs(loss - lref) <= 1e-5 * abs(lref)
+    assert np.max(np.abs(g - gref)) <= 1e-4 * np.max(np.abs(gref)) + 1e-7
+    t = torch()
+    act, probs = empty((n + 1,), t.int8), empty((n + 1, 4), t.float32)
+    mlp.infer(fd.data_ptr(), n, 0.6, act.data_ptr(), probs.data_ptr())
+    sync()
+    logit = oracle.mlp_forward(w16, f)[4]
+    ref = np.exp(logit - logit.max(1, keepdims=True))
+    ref /= ref.sum(1, keepdims=True)
+    # fp32 sums of 64 products and the hardware exponential
+    assert np.abs(probs.cpu().numpy()[:n] - ref).max() <= 2e-5
+    sure = np.abs(ref.max(1) - 0.6) > 1e-4
+    expected = np.where(ref.max(1) >= 0.6, ref.argmax(1), -1)
+    assert np.array_equal(act.cpu().numpy()[:n][sure], expected[sure])
+    assert act[n] == 0 and not probs[n].any()  # nothing past the end
+
+
 def test_gpu_training_recovers_the_decision_rule():
     f, labels, w = samples(40000, 2)
     mlp = gsn.Mlp(seed=5)
