@@ -23,6 +23,7 @@
 #include "kernels.h"
 #include "knn_kernels.h"
 #include "profile.h"
+#include "util/stream_buffer.h"
 
 struct gsn_renderer {
     gs_native::Renderer impl;
@@ -656,12 +657,13 @@ int gsn_trainer_evaluate_metrics(gsn_trainer* t, const gsn_camera* cameras, cons
 
 int gsn_spatial_permutation(const float* params, int count, uint32_t* perm, void* stream) {
     if (!params || !perm || count <= 0) return GSN_ERR_INVALID_ARGUMENT;
-    gs_native::SpatialOrder order;
-    order.SetStream(static_cast<cudaStream_t>(stream));
-    if (!order.Compute(params, count)) return GSN_ERR_CUDA;
-    if (cudaMemcpyAsync(perm, order.GetPermutation(), sizeof(uint32_t) * count, cudaMemcpyDeviceToDevice,
-                        static_cast<cudaStream_t>(stream)) != cudaSuccess ||
-        cudaStreamSynchronize(static_cast<cudaStream_t>(stream)) != cudaSuccess)
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    gs_native::StreamBuffer work(s);
+    if (!work.Allocate(gs_native::SpatialOrder::WorkspaceBytes(count))) return GSN_ERR_CUDA;
+    const uint32_t* order = gs_native::SpatialOrder::ComputeIn(work.get(), params, count, s);
+    if (!order) return GSN_ERR_CUDA;
+    if (cudaMemcpyAsync(perm, order, sizeof(uint32_t) * count, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
         return GSN_ERR_CUDA;
     return GSN_OK;
 }
@@ -674,12 +676,13 @@ int gsn_gather_gaussians(const float* src, float* dst, const uint32_t* perm, int
 int gsn_eval_metrics(const float* image, const uint8_t* target, int width, int height, double* out, void* stream) {
     if (!image || !target || !out || width <= 0 || height <= 0) return GSN_ERR_INVALID_ARGUMENT;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    gs_native::DeviceArray<double> workspace, metrics;
-    if (!workspace.Reserve(gsn::eval_metrics_workspace(width, height) / sizeof(double)) || !metrics.Reserve(4))
+    gs_native::StreamBuffer buffer(s);
+    if (!buffer.Allocate(4 * sizeof(double) + gsn::eval_metrics_workspace(width, height)))
         return GSN_ERR_OUT_OF_MEMORY;
-    const int st = gsn::launch_eval_metrics(image, target, width, height, workspace.get(), metrics.get(), s);
+    auto* metrics = reinterpret_cast<double*>(buffer.get());
+    const int st = gsn::launch_eval_metrics(image, target, width, height, metrics + 4, metrics, s);
     if (st != GSN_OK) return st;
-    if (cudaMemcpyAsync(out, metrics.get(), 4 * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    if (cudaMemcpyAsync(out, metrics, 4 * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return GSN_ERR_CUDA;
     return GSN_OK;

@@ -246,11 +246,11 @@ int launch_remap_moments(const int* parents, const float* prev_m, const float* p
 
 // ---------------------------------------------------------------- spatial order
 // Morton keys (30 bits, 10 per axis inside the bounding box of the finite
-// means; bounds: 6 ints of device scratch) for a spatial permutation of the
+// means; bounds: 6 words of device scratch) for a spatial permutation of the
 // Gaussians (spatial.cu); the row gather dst[r][i] = src[r][perm[i]] of a
 // parameter or moment block in either layout; and parents'[i] = parents[perm[i]]
 // (perm[i] itself when parents is null).
-int launch_morton_keys(const float* params, int n, int* bounds, uint32_t* keys, cudaStream_t stream);
+int launch_morton_keys(const float* params, int n, uint32_t* bounds, uint32_t* keys, cudaStream_t stream);
 int launch_gather_gaussians(const float* src, float* dst, const uint32_t* perm, int n, bool bf16_sh,
                             cudaStream_t stream);
 int launch_compose_parents(const int* parents, const uint32_t* perm, int n, int* out, cudaStream_t stream);

@@ -18,23 +18,28 @@ namespace gsn {
 
 namespace {
 
-// Order-preserving float <-> int map for atomicMin / atomicMax.
-__device__ __forceinline__ int ordered(float f) {
-    const int b = __float_as_int(f);
-    return b >= 0 ? b : b ^ 0x7FFFFFFF;
+// Order-preserving float <-> unsigned map for the min reductions.
+__device__ __forceinline__ uint32_t ordered(float f) {
+    const uint32_t b = __float_as_uint(f);
+    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
 }
-__device__ __forceinline__ float unordered(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7FFFFFFF); }
-
-__global__ void bounds_init(int* bounds) {
-    const int t = threadIdx.x;
-    if (t < 3) bounds[t] = 0x7FFFFFFF;
-    else if (t < 6) bounds[t] = static_cast<int>(0x80000000u);
+__device__ __forceinline__ float unordered(uint32_t u) {
+    return __uint_as_float((u & 0x80000000u) ? u & 0x7FFFFFFFu : ~u);
 }
 
+constexpr int kBoundsBlocks = 148 * 2;
+
+// bounds[0..2]: smallest ordered coordinates of the finite means; bounds[3..5]:
+// smallest complements (the largest coordinates), all initialised by one memset to
+// 0xFF. Six global atomics per block: with six per warp of 1,184 blocks the
+// atomics queued on one L2 line (42 us at 1.2M Gaussians).
 __global__ void __launch_bounds__(256) position_bounds(const float* __restrict__ params, int n,
-                                                       int* __restrict__ bounds) {
+                                                       uint32_t* __restrict__ bounds) {
+    __shared__ uint32_t s[6];
+    if (threadIdx.x < 6) s[threadIdx.x] = 0xFFFFFFFFu;
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+#pragma unroll 4
+    for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const float x = params[static_cast<int64_t>(a) * n + i];
@@ -44,21 +49,18 @@ __global__ void __launch_bounds__(256) position_bounds(const float* __restrict__
             }
         }
     }
+    __syncthreads();
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        const uint32_t l = __reduce_min_sync(0xffffffffu, ordered(lo[a]));
+        const uint32_t h = __reduce_min_sync(0xffffffffu, ~ordered(hi[a]));
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s[a], l);
+            atomicMin(&s[3 + a], h);
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(bounds + a, ordered(lo[a]));
-            atomicMax(bounds + 3 + a, ordered(hi[a]));
-        }
-    }
+    __syncthreads();
+    if (threadIdx.x < 6) atomicMin(bounds + threadIdx.x, s[threadIdx.x]);
 }
 
 __device__ __forceinline__ uint32_t spread10(uint32_t x) {
@@ -71,13 +73,14 @@ __device__ __forceinline__ uint32_t spread10(uint32_t x) {
 }
 
 __global__ void __launch_bounds__(256) morton_keys(const float* __restrict__ params, int n,
-                                                   const int* __restrict__ bounds, uint32_t* __restrict__ keys) {
+                                                   const uint32_t* __restrict__ bounds,
+                                                   uint32_t* __restrict__ keys) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t q[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float lo = unordered(bounds[a]), hi = unordered(bounds[3 + a]);
+        const float lo = unordered(bounds[a]), hi = unordered(~bounds[3 + a]);
         const float x = params[static_cast<int64_t>(a) * n + i];
         const float span = hi - lo;
         float f = span > 0.0f ? (x - lo) / span : 0.0f;
@@ -87,13 +90,30 @@ __global__ void __launch_bounds__(256) morton_keys(const float* __restrict__ par
     keys[i] = spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) gather_rows(const T* __restrict__ src, T* __restrict__ dst,
-                                                   const uint32_t* __restrict__ perm, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t row = static_cast<int64_t>(blockIdx.y) * n;
-    dst[row + i] = src[row + perm[i]];
+// Rows of 32-bit words: dst[r][i] = src[r][perm[i]]. A random permutation reads a
+// 32-byte sector per word, so the gather is bound by L2 sector traffic and by how
+// many of those reads are in flight: a thread takes kGatherItems Gaussians
+// (strided by the block, so loads of perm and stores stay coalesced) of kGatherRows
+// rows and issues all of its gathers together.
+constexpr int kGatherItems = 4, kGatherRows = 2;
+
+__global__ void __launch_bounds__(256) gather_rows(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
+                                                   const uint32_t* __restrict__ perm, int n, int rows) {
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * (256 * kGatherItems) + threadIdx.x;
+    const int row0 = blockIdx.y * kGatherRows;
+    uint32_t from[kGatherItems], v[kGatherRows][kGatherItems];
+#pragma unroll
+    for (int k = 0; k < kGatherItems; ++k) from[k] = first + 256 * k < n ? perm[first + 256 * k] : 0u;
+#pragma unroll
+    for (int r = 0; r < kGatherRows; ++r)
+#pragma unroll
+        for (int k = 0; k < kGatherItems; ++k)
+            v[r][k] = row0 + r < rows ? src[static_cast<int64_t>(row0 + r) * n + from[k]] : 0u;
+#pragma unroll
+    for (int r = 0; r < kGatherRows; ++r)
+#pragma unroll
+        for (int k = 0; k < kGatherItems; ++k)
+            if (row0 + r < rows && first + 256 * k < n) dst[static_cast<int64_t>(row0 + r) * n + first + 256 * k] = v[r][k];
 }
 
 __global__ void __launch_bounds__(256) compose_parents(const int* __restrict__ parents,
@@ -107,22 +127,24 @@ __global__ void __launch_bounds__(256) compose_parents(const int* __restrict__ p
 
 }  // namespace
 
-int launch_morton_keys(const float* params, int n, int* bounds, uint32_t* keys, cudaStream_t stream) {
+int launch_morton_keys(const float* params, int n, uint32_t* bounds, uint32_t* keys, cudaStream_t stream) {
     if (n <= 0) return GSN_OK;
     if (!params || !bounds || !keys) return GSN_ERR_INVALID_ARGUMENT;
-    bounds_init<<<1, 32, 0, stream>>>(bounds);
-    position_bounds<<<min(ceil_div(n, 256), 148 * 8), 256, 0, stream>>>(params, n, bounds);
+    if (cudaMemsetAsync(bounds, 0xFF, 6 * sizeof(uint32_t), stream) != cudaSuccess) return GSN_ERR_CUDA;
+    position_bounds<<<min(ceil_div(n, 256), kBoundsBlocks), 256, 0, stream>>>(params, n, bounds);
     morton_keys<<<ceil_div(n, 256), 256, 0, stream>>>(params, n, bounds, keys);
-    return launched(3);
+    return launched(2);
 }
 
 int launch_gather_gaussians(const float* src, float* dst, const uint32_t* perm, int n, bool bf16_sh,
                             cudaStream_t stream) {
     if (n <= 0) return GSN_OK;
     if (!src || !dst || !perm) return GSN_ERR_INVALID_ARGUMENT;
-    const unsigned blocks = static_cast<unsigned>(ceil_div(n, 256));
     // one 32-bit word per (physical row, Gaussian) in both layouts
-    gather_rows<float><<<dim3(blocks, bf16_sh ? kPrecisionPhysicalRows : kParams), 256, 0, stream>>>(src, dst, perm, n);
+    const int rows = bf16_sh ? kPrecisionPhysicalRows : kParams;
+    const dim3 grid(ceil_div(n, 256 * kGatherItems), ceil_div(rows, kGatherRows));
+    gather_rows<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(src), reinterpret_cast<uint32_t*>(dst),
+                                          perm, n, rows);
     return launched(1);
 }
 

@@ -7,19 +7,34 @@
 
 namespace gs_native {
 
-bool SpatialOrder::Compute(const float* params, int count) {
-    if (!params || count <= 0) return false;
-    const size_t n = static_cast<size_t>(count);
-    if (!keys_[0].Reserve(n) || !keys_[1].Reserve(n) || !ids_[0].Reserve(n) || !ids_[1].Reserve(n) ||
-        !bounds_.Reserve(6) || !sort_scratch_.Reserve(gsn::radix_sort_scratch_bytes(count)))
-        return false;
-    if (gsn::launch_morton_keys(params, count, bounds_.get(), keys_[0].get(), stream_) != GSN_OK) return false;
+namespace {
+size_t ArrayBytes(int count) { return (static_cast<size_t>(count) * sizeof(uint32_t) + 255) & ~static_cast<size_t>(255); }
+}  // namespace
+
+// keys and ids (two of each), the bounds, the sort's scratch
+size_t SpatialOrder::WorkspaceBytes(int count) {
+    return 4 * ArrayBytes(count) + 256 + gsn::radix_sort_scratch_bytes(count);
+}
+
+const uint32_t* SpatialOrder::ComputeIn(unsigned char* work, const float* params, int count, cudaStream_t stream) {
+    const size_t array = ArrayBytes(count);
+    uint32_t* keys[2] = {reinterpret_cast<uint32_t*>(work), reinterpret_cast<uint32_t*>(work + array)};
+    uint32_t* ids[2] = {reinterpret_cast<uint32_t*>(work + 2 * array), reinterpret_cast<uint32_t*>(work + 3 * array)};
+    auto* bounds = reinterpret_cast<uint32_t*>(work + 4 * array);
+    if (gsn::launch_morton_keys(params, count, bounds, keys[0], stream) != GSN_OK) return nullptr;
     bool in_alt = false;
-    const gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(sort_scratch_.get(), count);
-    if (gsn::launch_radix_sort(keys_[0].get(), ids_[0].get(), keys_[1].get(), ids_[1].get(), true, count, nullptr,
-                               0, 30, scratch, &in_alt, stream_) != GSN_OK)
-        return false;
-    perm_ = ids_[in_alt ? 1 : 0].get();
+    const gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(work + 4 * array + 256, count);
+    if (gsn::launch_radix_sort(keys[0], ids[0], keys[1], ids[1], true, count, nullptr, 0, 30, scratch, &in_alt,
+                               stream) != GSN_OK)
+        return nullptr;
+    return ids[in_alt ? 1 : 0];
+}
+
+bool SpatialOrder::Compute(const float* params, int count) {
+    if (!params || count <= 0 || !work_.Reserve(WorkspaceBytes(count))) return false;
+    const uint32_t* perm = ComputeIn(work_.get(), params, count, stream_);
+    if (!perm) return false;
+    perm_ = perm;
     count_ = count;
     return true;
 }

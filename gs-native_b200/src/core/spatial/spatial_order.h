@@ -20,6 +20,10 @@ public:
     // Permutation perm (device, count entries): new Gaussian i is old perm[i],
     // in ascending Morton order of the means (ties by old id).
     bool Compute(const float* params, int count);
+    // The same in a device workspace of the caller's (WorkspaceBytes, 256-byte
+    // aligned), which holds the result; null on failure.
+    static size_t WorkspaceBytes(int count);
+    static const uint32_t* ComputeIn(unsigned char* work, const float* params, int count, cudaStream_t stream);
     const uint32_t* GetPermutation() const { return perm_; }
     // Reorders the block in place (either layout) by the last permutation and
     // composes `parents` (device, nullable: identity) into GetParents():
@@ -31,9 +35,8 @@ public:
 
 private:
     cudaStream_t stream_ = nullptr;
-    DeviceArray<uint32_t> keys_[2], ids_[2];
-    DeviceArray<uint8_t> sort_scratch_;
-    DeviceArray<int> bounds_, parents_;
+    DeviceArray<unsigned char> work_;
+    DeviceArray<int> parents_;
     DeviceArray<float> block_;
     const uint32_t* perm_ = nullptr;
     int count_ = 0;

@@ -3,6 +3,8 @@
 
 #include <atomic>
 
+#include "util/stream_buffer.h"
+
 namespace gs_native {
 
 namespace {
@@ -14,7 +16,14 @@ void SetDeviceAllocHook(DeviceAllocFn fn) { g_alloc_hook.store(fn); }
 cudaError_t DeviceAlloc(void** ptr, size_t bytes) {
     DeviceAllocFn fn = g_alloc_hook.load();
     if (fn) return fn(ptr, bytes);
-    return cudaMalloc(ptr, bytes);
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        // what the scratch pools keep may be what is missing
+        cudaGetLastError();
+        ReleaseStreamPools();
+        e = cudaMalloc(ptr, bytes);
+    }
+    return e;
 }
 
 }  // namespace gs_native

@@ -59,6 +59,36 @@ def test_spatial_permutation_is_morton_sort_and_gathers():
     assert np.array_equal(back, ref)
 
 
+@pytest.mark.parametrize("n", [1, 2, 255, 1023, 1025, 4097])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_permutation_and_gather_at_the_edges_of_blocks(n, bf16):
+    t = torch()
+    params = scenes.random_gaussians(max(n, 2), n, mean_sigma=2.0)[:, :n].copy()
+    if n > 2:
+        params[1, n // 2], params[0, 1] = np.nan, np.inf  # outside the bounding box of the finite means
+    p = dev(params)
+    perm = t.full((n + 1,), -1, dtype=t.int32, device="cuda")
+    gsn.spatial_permutation(p.data_ptr(), n, perm.data_ptr())
+    block = gsn.to_precision_layout(params, t) if bf16 else p
+    rows = 34 if bf16 else 58
+    out = t.full((rows * n + 1,), -7.0, dtype=t.float32, device="cuda")
+    gsn.gather_gaussians(block.data_ptr(), out.data_ptr(), perm.data_ptr(), n, bf16_sh=bf16)
+    sync()
+    pm = perm.cpu().numpy()
+    assert np.array_equal(np.sort(pm[:n]), np.arange(n)) and pm[n] == -1 and out[-1] == -7.0
+    words = block.view(t.int32).cpu().numpy().reshape(rows, n)
+    assert np.array_equal(out[:-1].view(t.int32).cpu().numpy().reshape(rows, n), words[:, pm[:n]])
+    if n > 2:
+        finite = np.isfinite(params[:3]).all(0)
+        pos, ok = params[:3], np.isfinite(params[:3])
+        lo = np.where(ok, pos, np.inf).min(1, keepdims=True).astype(np.float32)
+        hi = np.where(ok, pos, -np.inf).max(1, keepdims=True).astype(np.float32)
+        f = np.where(ok, np.clip((np.where(ok, pos, 0) - lo) / (hi - lo), 0, 1), 1).astype(np.float32)
+        q = (f * np.float32(1023.0) + np.float32(0.5)).astype(np.uint64)
+        keys = (_spread(q[0]) | (_spread(q[1]) << np.uint64(1)) | (_spread(q[2]) << np.uint64(2))).astype(np.int64)
+        assert (np.diff(keys[pm[:n]]) >= 0).all() and (~finite).sum() == 2
+
+
 def test_permuted_model_renders_the_same_image():
     t = torch()
     params = scenes.random_gaussians(40000, 5, mean_sigma=2.0)
