@@ -6,11 +6,13 @@
 // Persistent kernel: CTAs take (view, tile) work items from a device counter,
 // so views of different sizes share the machine without a launch per view and
 // the tail of one view overlaps the next. The per-tile blend is the plain
-// renderer's (front-to-back, conservative alpha-box culling per warp strip, the
-// alpha floor before expf, early stop when the tile is saturated) with the
-// same per-pixel arithmetic (renderer.cu:273-338), generalised to TW x TH tiles
-// and THREADS threads: warp w owns a strip of TH / warps rows, lane l the
-// column l % TW and the rows (l / TW) + p * (32 / TW) of that strip.
+// renderer's (front-to-back, records culled per warp region by raster_common.cuh
+// region_hit, the alpha floor before expf, early stop when the tile is saturated)
+// with the same per-pixel arithmetic (renderer.cu:273-338), generalised to TW x TH
+// tiles and THREADS threads: a warp owns a region of the tile, 8 pixels wide where
+// the tile's warps can share it so (an ellipse misses more of a square region than
+// of a flat one) and the whole width otherwise; lane l has the region's column
+// l % W and its rows l / W + p * (32 / W).
 #include <algorithm>
 
 #include "raster_common.cuh"
@@ -26,24 +28,27 @@ constexpr int kBatch = 128;  // records staged per round
 template <int TW, int TH, int THREADS>
 struct Geometry {
     static constexpr int kWarps = THREADS / 32;
-    static constexpr int kStripRows = TH / kWarps;       // rows per warp
-    static constexpr int kRowsPerPass = 32 / TW;         // rows covered by one warp-wide pixel set
-    static constexpr int kPix = kStripRows / kRowsPerPass;  // pixels per thread
-    static_assert(kPix >= 1 && kStripRows % kRowsPerPass == 0, "tile shape / threads combination");
+    static constexpr int kColumns = TW / 8 <= kWarps && TH * TW / kWarps <= 64 ? TW / 8 : 1;  // regions side by side
+    static constexpr int kWidth = TW / kColumns;                // a warp's region
+    static constexpr int kHeight = TH / (kWarps / kColumns);
+    static constexpr int kRowsPerPass = 32 / kWidth;            // rows covered by one warp-wide pixel set
+    static constexpr int kPix = kHeight / kRowsPerPass;         // pixels per thread
+    static_assert(kPix >= 1 && kHeight % kRowsPerPass == 0 && kWarps % kColumns == 0, "tile shape / threads");
 };
 
 template <int TW, int TH, int THREADS>
-__device__ __forceinline__ void blend_tile(const MultiView& v, int tile, float2* s_mean, float4* s_conic,
-                                           float3* s_color, float4* s_box, float* s_floor) {
+__device__ __forceinline__ void blend_tile(const MultiView& v, int tile, float4* s_head, float4* s_conic,
+                                           float2* s_tail, float* s_cull) {
     using G = Geometry<TW, TH, THREADS>;
     constexpr int P = G::kPix;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int tx = tile % v.tiles_x, ty = tile / v.tiles_x;
-    const int px = tx * TW + lane % TW;
-    const int row0 = ty * TH + warp * G::kStripRows + lane / TW;
+    const int rx = tx * TW + warp % G::kColumns * G::kWidth, ry = ty * TH + warp / G::kColumns * G::kHeight;
+    const int px = rx + lane % G::kWidth;
+    const int row0 = ry + lane / G::kWidth;
     const float fx = static_cast<float>(px);
-    const float sx0 = static_cast<float>(tx * TW), sx1 = sx0 + (TW - 1);
-    const float sy0 = static_cast<float>(ty * TH + warp * G::kStripRows), sy1 = sy0 + (G::kStripRows - 1);
+    const float sx0 = static_cast<float>(rx), sx1 = sx0 + (G::kWidth - 1);
+    const float sy0 = static_cast<float>(ry), sy1 = sy0 + (G::kHeight - 1);
     float fy[P], T[P];
     float3 C[P];
     bool done[P];
@@ -74,54 +79,53 @@ __device__ __forceinline__ void blend_tile(const MultiView& v, int tile, float2*
                 const float* cp = reinterpret_cast<const float*>(v.colors) + 3ull * id;
                 c = make_float3(__ldg(cp), __ldg(cp + 1), __ldg(cp + 2));
             }
-            s_mean[slot] = mean;
+            s_head[slot] = make_float4(mean.x, mean.y, c.x, c.y);
             s_conic[slot] = q;
-            s_color[slot] = c;
-            s_box[slot] = alpha_box(mean, q);
-            s_floor[slot] = alpha_floor(q.w);
+            s_tail[slot] = make_float2(c.z, alpha_floor(q.w));
+            s_cull[slot] = cull_limit(mean, q);
         }
         __syncthreads();
         const int batch = static_cast<int>(min(static_cast<int64_t>(kBatch), end - base));
 #pragma unroll 1
         for (int k = 0; k < kBatch / 32; ++k) {
             const int jl = k * 32 + lane;
-            uint32_t m = __ballot_sync(0xffffffffu, jl < batch && box_hits(s_box[jl], sx0, sx1, sy0, sy1));
-            while (m) {
-                bool all = true;
+            bool hit = jl < batch;
+            if (hit) {
+                const float4 q = s_conic[jl];
+                hit = region_hit(make_float2(s_head[jl].x, s_head[jl].y), q.x, 2.0f * q.y, q.z, s_cull[jl], sx0, sx1, sy0, sy1);
+            }
+            uint32_t m = __ballot_sync(0xffffffffu, hit);
+            bool all = true;
 #pragma unroll
-                for (int p = 0; p < P; ++p) all = all && done[p];
-                if (all) break;
-                const int j = k * 32 + __ffs(m) - 1;
-                m &= m - 1;
-                const float2 mu = s_mean[j];
+            for (int p = 0; p < P; ++p) all = all && done[p];
+            if (__all_sync(0xffffffffu, all)) break;
+            while (m) {  // the same for every lane
+                const uint32_t bit = m & (0u - m);
+                m ^= bit;
+                const int j = k * 32 + 31 - __clz(bit);
+                const float4 head = s_head[j];
                 const float4 q = s_conic[j];
-                const float lim = s_floor[j];
-                const float3 c = s_color[j];
-                const float dx = mu.x - fx;
-                float pw[P];
-                bool act[P];
-                bool any = false;
+                const float2 tail = s_tail[j];
+                const float dx = head.x - fx;
+                const Power power(q, dx);
+                // every pixel evaluated branch-free, as in the single-view blend
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
-                    const float dy = mu.y - fy[p];
-                    pw[p] = -0.5f * (q.x * dx * dx + q.z * dy * dy) - q.y * dx * dy;
-                    act[p] = !done[p] && !(pw[p] > 0.0f) && !(pw[p] < lim);
-                    any |= act[p];
-                }
-                if (!any) continue;
-#pragma unroll
-                for (int p = 0; p < P; ++p) {
-                    const float alpha = fminf(kAlphaMax, q.w * expf(pw[p]));
-                    bool take = act[p] && !(alpha < kAlphaMin);
+                    const float pw = power.at(head.y - fy[p]);
+                    const bool act = !done[p] && !(pw > 0.0f) && !(pw < tail.y);
+                    const float alpha = fminf(kAlphaMax, gaussian_weight<false>(q.w, pw));
+                    bool take = act && !(alpha < kAlphaMin);
                     const float nextT = T[p] * (1.0f - alpha);
                     const bool stop = take && nextT < kTransmittanceMin;
                     done[p] = done[p] || stop;
                     take = take && !stop;
                     const float w = alpha * T[p];
-                    C[p].x = take ? C[p].x + c.x * w : C[p].x;
-                    C[p].y = take ? C[p].y + c.y * w : C[p].y;
-                    C[p].z = take ? C[p].z + c.z * w : C[p].z;
-                    T[p] = take ? nextT : T[p];
+                    if (take) {
+                        C[p].x = fmaf(head.z, w, C[p].x);
+                        C[p].y = fmaf(head.w, w, C[p].y);
+                        C[p].z = fmaf(tail.x, w, C[p].z);
+                        T[p] = nextT;
+                    }
                 }
             }
         }
@@ -140,11 +144,10 @@ __device__ __forceinline__ void blend_tile(const MultiView& v, int tile, float2*
 
 template <int TW, int TH, int THREADS>
 __global__ void __launch_bounds__(THREADS) multiview_kernel(MultiViewArgs a) {
-    __shared__ float2 s_mean[kBatch];
-    __shared__ float4 s_conic[kBatch];
-    __shared__ float3 s_color[kBatch];
-    __shared__ float4 s_box[kBatch];
-    __shared__ float s_floor[kBatch];
+    __shared__ float4 s_head[kBatch];   // mean, red and green
+    __shared__ float4 s_conic[kBatch];  // conic and opacity
+    __shared__ float2 s_tail[kBatch];   // blue, alpha floor
+    __shared__ float s_cull[kBatch];    // cull_limit
     __shared__ int s_item;
     while (true) {
         if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
@@ -154,7 +157,8 @@ __global__ void __launch_bounds__(THREADS) multiview_kernel(MultiViewArgs a) {
         if (item >= a.total_tiles) break;
         int v = 0;
         while (v + 1 < a.view_count && a.tile_prefix[v + 1] <= item) ++v;
-        blend_tile<TW, TH, THREADS>(a.views[v], item - a.tile_prefix[v], s_mean, s_conic, s_color, s_box, s_floor);
+        blend_tile<TW, TH, THREADS>(a.views[v], item - a.tile_prefix[v], s_head, s_conic,
+                                    s_tail, s_cull);
     }
 }
 

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kRasterThreads, 12) raster_backward_kernel(Ras
 #pragma unroll
                     for (int i = 0; i < 9; ++i) v[i] = acc[i].x + acc[i].y;
                 } else {
-                    const Power<false> power(q, dx);
+                    const Power power(q, dx);
                     const float lim = s_floor[j];
 #pragma unroll
                     for (int p = 0; p < kPixPerThread; ++p) {
