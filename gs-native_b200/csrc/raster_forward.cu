@@ -93,6 +93,7 @@ template <bool kFast, bool kCount>
 __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterForwardArgs a) {
     pdl_begin();
     __shared__ __align__(16) Record s_rec[kRasterBatch];
+    __shared__ int s_bound;
 
     const int t = threadIdx.x;
     const int lane = t & 31;
@@ -130,6 +131,14 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
 #pragma unroll
         for (int p = 0; p < kForwardPix; ++p) mine = mine && done[p];
         if (__syncthreads_and(mine)) break;
+        if (a.checkpoints && base > begin) {
+            float4* state = a.checkpoints +
+                            checkpoint_slot(begin, tile, static_cast<int>(base - begin)) * kTilePixels;
+            const int in_tile = (8 * (warp >> 1) + (lane >> 3)) * kTile + 8 * (warp & 1) + (lane & 7);
+#pragma unroll
+            for (int p = 0; p < kForwardPix; ++p)
+                state[in_tile + 4 * p * kTile] = make_float4(T[p], C[p].x, C[p].y, C[p].z);
+        }
         stage<kFast>(next, s_rec + t);
         __syncthreads();
         next = fetch(a, base + kRasterBatch + t, end);
@@ -226,6 +235,17 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
             }
         }
     }
+    if (a.tile_bounds) {
+        int most = 0;
+#pragma unroll
+        for (int p = 0; p < kForwardPix; ++p) most = max(most, consumed[p]);
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (t == 0) s_bound = 0;
+        __syncthreads();
+        if (lane == 0) atomicMax(&s_bound, most);
+        __syncthreads();
+        if (t == 0) a.tile_bounds[tile] = s_bound;
+    }
     if (kCount) {
         const unsigned long long warp_pairs = __reduce_add_sync(0xffffffffu, pairs);
         if (lane == 0 && warp_pairs) atomicAdd(a.pair_count, warp_pairs);
@@ -244,6 +264,10 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
 }
 
 }  // namespace
+
+size_t checkpoint_blocks(int64_t records, int tiles) {
+    return static_cast<size_t>(records) / kSegment + static_cast<size_t>(tiles);
+}
 
 int launch_raster_forward(const RasterForwardArgs& a, cudaStream_t stream) {
     int64_t tiles = static_cast<int64_t>(a.cam.tile_count_x) * a.cam.tile_count_y;

@@ -80,7 +80,9 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     sh_degree = std::clamp(sh_degree, 0, 3);
     if (!ReserveGaussians(count)) return false;
     if (static_cast<size_t>(tile_count) > tile_capacity_) {
-        if (!tile_offsets_.Reserve(static_cast<size_t>(tile_count) + 1)) return false;
+        if (!tile_offsets_.Reserve(static_cast<size_t>(tile_count) + 1) ||
+            !tile_bounds_.Reserve(static_cast<size_t>(tile_count)))
+            return false;
         tile_capacity_ = static_cast<size_t>(tile_count);
     }
     const size_t pixels = static_cast<size_t>(camera.width_) * camera.height_;
@@ -140,7 +142,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
             cudaSuccess)
             return false;
     }
-    return Blend(cam, background, image);
+    return Blend(cam, background, image, tile_count);
 }
 
 // Per-tile lists by emitting the records in depth order and stable-sorting
@@ -208,8 +210,12 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 }
 
 // The per-tile blend of the ordered records.
-bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image) {
+bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
+    checkpoints_used_ = tile_count <= gsn::kCheckpointTiles;
+    if (checkpoints_used_ &&
+        !checkpoints_.Reserve(gsn::checkpoint_blocks(record_capacity_, tile_count) * GSN_TILE_SIZE * GSN_TILE_SIZE))
+        return false;
     gsn::RasterForwardArgs ra;
     ra.tile_ids = sorted_ids_;
     ra.tile_offsets = tile_offsets_.get();
@@ -224,6 +230,8 @@ bool Renderer::Blend(const gsn_camera& cam, const float* background, float* imag
     ra.record_warps = record_warps_.get();
     ra.record_words = record_words_;
     ra.fast = fast_blend_;
+    ra.tile_bounds = tile_bounds_.get();
+    ra.checkpoints = checkpoints_used_ ? checkpoints_.get() : nullptr;
     ra.pair_count = pair_counter_;
     if (record_warps_.get() &&
         cudaMemsetAsync(record_warps_.get(), 0, 2 * static_cast<size_t>(record_words_) * sizeof(uint32_t), s) !=

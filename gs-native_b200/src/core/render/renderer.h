@@ -90,6 +90,11 @@ public:
     // forward pass. The backward pass skips the others.
     const uint32_t* GetRecordWarps() const { return record_warps_.get(); }
     int64_t GetRecordWords() const { return record_words_; }
+    // Per tile of the last frame, the largest contributor count of its pixels.
+    const int* GetTileBounds() const { return tile_bounds_.get(); }
+    // Per-pixel blend states inside long lists, kept for frames of few tiles (null
+    // otherwise): the backward pass starts its segments from them.
+    const float4* GetCheckpoints() const { return checkpoints_used_ ? checkpoints_.get() : nullptr; }
     const int* GetRecordCountDevice() const { return counters_.get(); }
     const int* GetOverflowFlag() const { return counters_.get() + 1; }
     int64_t GetRecordCapacity() const { return record_capacity_; }
@@ -107,7 +112,7 @@ private:
     int64_t record_capacity_ = 0;
     bool OrderBySort(const uint32_t* by_depth, const int* visible, int count, const CameraParams& camera,
                      int tile_count, int64_t* records_out);
-    bool Blend(const gsn_camera& cam, const float* background, float* image);
+    bool Blend(const gsn_camera& cam, const float* background, float* image, int tile_count);
 
     bool fixed_capacity_ = false;
     const gsn_camera* device_camera_ = nullptr;
@@ -137,6 +142,9 @@ private:
     uint32_t* sorted_ids_ = nullptr;
     DeviceArray<int> contributors_;
     DeviceArray<uint32_t> record_warps_;
+    DeviceArray<int> tile_bounds_;
+    DeviceArray<float4> checkpoints_;
+    bool checkpoints_used_ = false;
     int64_t record_words_ = 0;
     size_t pixel_capacity_ = 0;
     DeviceArray<unsigned char> sort_scratch_;

@@ -133,6 +133,8 @@ bool Solver::ComputeScreenGradients(const CameraParams& camera, const Renderer& 
     a.contributors = renderer.GetContributors();
     a.record_warps = renderer.GetRecordWarps();
     a.record_words = renderer.GetRecordWords();
+    a.tile_bounds = renderer.GetTileBounds();
+    a.checkpoints = renderer.GetCheckpoints();
     a.fast = renderer.GetFastBlend();
     a.cam = AsGsnCamera(camera);
     a.grad_out = screen_.get();
