@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(1024) levels_kernel(KnnTree tree, float4* lo, 
 // Squared distance of the box [plo, phi] (a point when equal) to a node's box.
 // Each difference, square and sum is monotonic under rounding, so the distance of
 // a box is never above that of a point inside it.
-__device__ __forceinline__ float box_distance(float3 plo, float3 phi, float3 lo, float3 hi) {
+__device__ __forceinline__ float box_distance(float3 plo, float3 phi, float4 lo, float4 hi) {
     const float x = fmaxf(fmaxf(lo.x - phi.x, plo.x - hi.x), 0.0f);
     const float y = fmaxf(fmaxf(lo.y - phi.y, plo.y - hi.y), 0.0f);
     const float z = fmaxf(fmaxf(lo.z - phi.z, plo.z - hi.z), 0.0f);
@@ -277,20 +277,14 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
     int level = tree.levels - 1, base = 0;
     uint32_t masks[kMaxLevels];
     int bases[kMaxLevels];
-    // this lane's child of `base`'s node at `level`: its box stays in registers, so that
-    // testing a child against every lane's point is six shuffles and no load
-    float3 clo = make_float3(0.0f, 0.0f, 0.0f), chi = clo;
-    auto load_children = [&]() {
-        const int child = min(base + lane, tree.count[level] - 1);
-        const float4 l = lo[tree.offset[level] + child], h = hi[tree.offset[level] + child];
-        clo = make_float3(l.x, l.y, l.z);
-        chi = make_float3(h.x, h.y, h.z);
-    };
-    // the children whose box is within the warp's largest bound of the warp's box
+    // children of `base`'s node at `level` whose box is within the warp's largest bound
     auto candidates = [&]() {
-        load_children();
         const float widest = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(bound, 0.0f))));
-        return __ballot_sync(kAll, base + lane < tree.count[level] && box_distance(qlo, qhi, clo, chi) <= widest);
+        const int child = base + lane;
+        bool near = false;
+        if (child < tree.count[level])
+            near = box_distance(qlo, qhi, lo[tree.offset[level] + child], hi[tree.offset[level] + child]) <= widest;
+        return __ballot_sync(kAll, near);
     };
     uint32_t mask = candidates();
     while (true) {
@@ -298,7 +292,6 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
             if (++level >= tree.levels) break;
             mask = masks[level];
             base = bases[level];
-            if (mask) load_children();
             continue;
         }
         // the child that holds this warp's own points first: its neighbours tighten the bounds
@@ -307,9 +300,9 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
         mask &= ~(1u << c);
         const int node = base + c;
         if (level == 0 && node / (32 / kBucket) == warp) continue;  // the warp's own points, already done
-        const float3 l = make_float3(__shfl_sync(kAll, clo.x, c), __shfl_sync(kAll, clo.y, c), __shfl_sync(kAll, clo.z, c));
-        const float3 h = make_float3(__shfl_sync(kAll, chi.x, c), __shfl_sync(kAll, chi.y, c), __shfl_sync(kAll, chi.z, c));
-        if (!__any_sync(kAll, box_distance(p, p, l, h) <= bound)) continue;
+        if (!__any_sync(kAll, box_distance(p, p, lo[tree.offset[level] + node], hi[tree.offset[level] + node]) <=
+                                  bound))
+            continue;
         if (level > 0) {
             masks[level] = mask;
             bases[level] = base;
