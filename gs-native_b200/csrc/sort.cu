@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <atomic>
 #include <mutex>
 
 namespace gsn {
@@ -26,8 +27,17 @@ constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 // 12 keys per thread measured fastest (8: tile sort 0.139 ms, 12: 0.128 ms, 16:
 // 0.136 ms at 7.2M records): longer scatter runs against fewer CTAs per SM
-constexpr int kSortItems = 12;                      // per thread
+constexpr int kSortItems = 12;                         // per thread
 constexpr int kSortChunk = kSortThreads * kSortItems;  // 3072 keys per block
+// Up to kMidCount keys the passes take 4 keys per thread instead: such a sort has
+// fewer blocks than SMs, so a pass lasts as long as one block's chain of ranking
+// steps, which a third of the keys makes a third as long.
+constexpr int kMidItems = 4;
+constexpr int kMidCount = 256 * kSortThreads * kMidItems;
+// Up to kSmallCount keys one block does the whole sort in shared memory.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallItems = 8;
+constexpr int kSmallCount = kSmallThreads * kSmallItems;
 constexpr int kBins = 256;
 // Each pass's digit totals are kept as kTotalCopies partial copies, one 1 KB row
 // apart, and a block adds into copy blockIdx % kTotalCopies: the thousands of
@@ -50,7 +60,7 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 // Per-block digit histogram of one digit of at most 8 bits (digits <= mask).
-template <bool kDrop>
+template <bool kDrop, int kItems>
 __global__ void __launch_bounds__(kSortThreads) radix_upsweep(const uint32_t* __restrict__ keys,
                                                               const int* n_dev, int n_host, int bit, uint32_t mask,
                                                               uint32_t* __restrict__ block_hist,
@@ -59,21 +69,21 @@ __global__ void __launch_bounds__(kSortThreads) radix_upsweep(const uint32_t* __
     pdl_begin();
     __shared__ uint32_t hist[kSortWarps][kBins];
     const int n = load_count(n_dev, n_host);
-    const int64_t start = static_cast<int64_t>(blockIdx.x) * kSortChunk;
+    const int64_t start = static_cast<int64_t>(blockIdx.x) * kItems * kSortThreads;
     if (start >= n) return;
-    const int64_t end = min(static_cast<int64_t>(n), start + kSortChunk);
+    const int64_t end = min(static_cast<int64_t>(n), start + kItems * kSortThreads);
     const int warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kSortWarps * kBins; i += kSortThreads) (&hist[0][0])[i] = 0;
     __syncthreads();
     // the chunk's loads first, then the shared-memory counts
-    uint32_t key[kSortItems];
+    uint32_t key[kItems];
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         const int64_t idx = start + k * kSortThreads + threadIdx.x;
         key[k] = idx < end ? __ldg(keys + idx) : kSortSentinel;
     }
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         const int64_t idx = start + k * kSortThreads + threadIdx.x;
         if (idx < end && (!kDrop || key[k] != kSortSentinel)) atomicAdd(&hist[warp][(key[k] >> bit) & mask], 1u);
     }
@@ -97,7 +107,7 @@ __device__ __forceinline__ uint32_t digit_sum(const uint32_t* __restrict__ digit
 
 // One block per digit: exclusive scan of that digit's per-block counts, offset by
 // the number of keys with a smaller digit.
-__global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int n_host,
+__global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int n_host, int chunk,
                                                            uint32_t* __restrict__ block_hist,
                                                            size_t hist_stride,
                                                            const uint32_t* __restrict__ digit_total) {
@@ -105,7 +115,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int
     __shared__ uint32_t warp_sums[kSortWarps];
     __shared__ uint32_t carry;
     const int n = load_count(n_dev, n_host);
-    const int blocks = ceil_div(n, kSortChunk);
+    const int blocks = ceil_div(n, chunk);
     const int d = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // base = sum of totals of smaller digits
@@ -161,14 +171,14 @@ __global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int
     }
 }
 
-// Stable scatter. Warp w owns the w-th 384-key slice of the block's chunk and
-// walks it in 32-key steps; eight ballots (one per digit bit) find the lanes with
+// Stable scatter. Warp w owns the w-th slice (32 kItems keys) of the block's chunk
+// and walks it in 32-key steps; eight ballots (one per digit bit) find the lanes with
 // an equal digit inside a step, and
 // warp-private counters carry the rank across steps, which keeps the original
 // order among equal digits. The ranked keys are first placed digit-sorted in
 // shared memory and then written out linearly, so each warp store covers a run
 // of consecutive addresses of one digit bucket instead of 32 scattered words.
-template <bool kIdentityValues, bool kDrop>
+template <bool kIdentityValues, bool kDrop, int kItems>
 __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ values_in,
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ values_out, const int* n_dev, int n_host,
@@ -177,12 +187,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
     __shared__ uint32_t counts[kSortWarps][kBins];
     __shared__ uint32_t global_base[kBins];
     __shared__ uint32_t local_base[kBins];
-    __shared__ uint32_t s_keys[kSortChunk];
-    __shared__ uint32_t s_vals[kSortChunk];
+    __shared__ uint32_t s_keys[(kItems * kSortThreads)];
+    __shared__ uint32_t s_vals[(kItems * kSortThreads)];
     const int n = load_count(n_dev, n_host);
-    const int64_t start = static_cast<int64_t>(blockIdx.x) * kSortChunk;
+    const int64_t start = static_cast<int64_t>(blockIdx.x) * (kItems * kSortThreads);
     if (start >= n) return;
-    const int64_t end = min(static_cast<int64_t>(n), start + kSortChunk);
+    const int64_t end = min(static_cast<int64_t>(n), start + (kItems * kSortThreads));
     __shared__ int s_total;  // keys of this chunk that are written (all but dropped sentinels)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kSortWarps * kBins; i += kSortThreads) (&counts[0][0])[i] = 0;
@@ -192,12 +202,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
     __syncthreads();
 
     const uint32_t lt = lanemask_lt();
-    const int64_t slice = start + static_cast<int64_t>(warp) * (kSortItems * 32);
-    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+    const int64_t slice = start + static_cast<int64_t>(warp) * (kItems * 32);
+    uint32_t key[kItems], val[kItems], rank[kItems];
     // all of the slice's loads first, so they are in flight together (the
     // warp-synchronous ranking below would otherwise wait for each step's pair)
 #pragma unroll
-    for (int s = 0; s < kSortItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         const int64_t idx = slice + s * 32 + lane;
         const bool valid = idx < end;
         key[s] = valid ? keys_in[idx] : 0u;
@@ -205,7 +215,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
         else val[s] = valid ? values_in[idx] : 0u;
     }
 #pragma unroll
-    for (int s = 0; s < kSortItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         bool valid = slice + s * 32 + lane < end;
         if (kDrop) valid = valid && key[s] != kSortSentinel;
         uint32_t digit = valid ? ((key[s] >> bit) & mask) : 0u;
@@ -257,7 +267,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
     __syncthreads();
     const int total = kDrop ? s_total : static_cast<int>(end - start);
 #pragma unroll
-    for (int s = 0; s < kSortItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         if (rank[s] == 0xFFFFFFFFu) continue;
         uint32_t digit = (key[s] >> bit) & mask;
         uint32_t pos = local_base[digit] + counts[warp][digit] + rank[s];
@@ -287,6 +297,132 @@ __global__ void radix_kept(const uint32_t* __restrict__ digit_total, int* __rest
         uint32_t s = 0;
         for (int w = 0; w < kSortWarps; ++w) s += part[w];
         *kept = static_cast<int>(s);
+    }
+}
+
+// The whole sort of at most kSmallCount pairs in one block: the same passes, digits
+// and stable ranking, with the pairs in shared memory between them. Three launches per
+// pass cost 15 us however few the keys are: 62 us for the 32-bit sort of 4,096 keys,
+// which takes 25 us here.
+struct SmallSmem {
+    uint32_t keys[kSmallCount], vals[kSmallCount];
+    uint16_t counts[kSmallThreads / 32][kBins];  // a warp's keys per digit, then where its first goes
+    uint32_t digit_base[kBins];
+    uint32_t warp_total[kBins / 32];
+};
+
+__global__ void __launch_bounds__(kSmallThreads) radix_small(const uint32_t* keys_in, const uint32_t* values_in,
+                                                             uint32_t* keys_out, uint32_t* values_out,
+                                                             const int* n_dev, int n_host, int begin_bit,
+                                                             int end_bit, bool identity, int* kept) {
+    pdl_begin();
+    extern __shared__ __align__(16) unsigned char smem[];
+    SmallSmem& sm = *reinterpret_cast<SmallSmem*>(smem);
+    constexpr int kWarps = kSmallThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt = lanemask_lt();
+    int n = load_count(n_dev, n_host);
+    uint32_t key[kSmallItems], val[kSmallItems], rank[kSmallItems];
+    const int passes = (end_bit - begin_bit + 7) / 8, width = end_bit - begin_bit;
+    bool drop = kept != nullptr;
+    int bit = begin_bit;
+    for (int p = 0; p < passes; ++p) {
+        const int digit_bits = width / passes + (p < width % passes ? 1 : 0);
+        const uint32_t mask = (1u << digit_bits) - 1u;
+        const int items = (n + kSmallThreads - 1) / kSmallThreads;
+        const int slice = warp * items * 32;
+#pragma unroll
+        for (int k = 0; k < kSmallItems; ++k) {
+            const int i = slice + k * 32 + lane;
+            if (k < items && i < n) {
+                key[k] = p == 0 ? keys_in[i] : sm.keys[i];
+                val[k] = p == 0 ? (identity ? static_cast<uint32_t>(i) : values_in[i]) : sm.vals[i];
+            }
+        }
+        for (int i = lane; i < kBins; i += 32) sm.counts[warp][i] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kSmallItems; ++k) {
+            if (k >= items) break;
+            bool valid = slice + k * 32 + lane < n;
+            if (drop) valid = valid && key[k] != kSortSentinel;
+            const uint32_t digit = valid ? (key[k] >> bit) & mask : 0u;
+            uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                if (b >= digit_bits) break;
+                const uint32_t bal = __ballot_sync(0xffffffffu, (digit >> b) & 1u);
+                peers &= ((digit >> b) & 1u) ? bal : ~bal;
+            }
+            const uint32_t before = valid ? sm.counts[warp][digit] : 0u;
+            __syncwarp();
+            rank[k] = valid ? before + __popc(peers & lt) : 0xFFFFFFFFu;
+            if (valid && (peers & lt) == 0) sm.counts[warp][digit] = static_cast<uint16_t>(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        {   // four threads per digit: exclusive prefix over the warps, then over the digits
+            const int d = threadIdx.x >> 2, quarter = threadIdx.x & 3;
+            uint32_t sum = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps / 4; ++w) sum += sm.counts[quarter * (kWarps / 4) + w][d];
+            uint32_t inc = sum;
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o, 4);
+                if (quarter >= o) inc += y;
+            }
+            uint32_t run = inc - sum;
+#pragma unroll
+            for (int w = 0; w < kWarps / 4; ++w) {
+                const uint32_t c = sm.counts[quarter * (kWarps / 4) + w][d];
+                sm.counts[quarter * (kWarps / 4) + w][d] = static_cast<uint16_t>(run);
+                run += c;
+            }
+            if (quarter == 3) sm.digit_base[d] = run;  // the digit's total
+        }
+        __syncthreads();
+        uint32_t mine = 0, total = 0;
+        if (threadIdx.x < kBins) {
+            total = sm.digit_base[threadIdx.x];
+            mine = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, mine, o);
+                if (lane >= o) mine += y;
+            }
+            if (lane == 31) sm.warp_total[warp] = mine;
+        }
+        __syncthreads();
+        uint32_t all = 0;
+#pragma unroll
+        for (int w = 0; w < kBins / 32; ++w) {
+            if (threadIdx.x < kBins && w < warp) mine += sm.warp_total[w];
+            all += sm.warp_total[w];
+        }
+        if (threadIdx.x < kBins) sm.digit_base[threadIdx.x] = mine - total;
+        __syncthreads();
+        const bool last = p + 1 == passes;
+#pragma unroll
+        for (int k = 0; k < kSmallItems; ++k) {
+            if (k >= items || slice + k * 32 + lane >= n || rank[k] == 0xFFFFFFFFu) continue;
+            const uint32_t digit = (key[k] >> bit) & mask;
+            const uint32_t pos = sm.digit_base[digit] + sm.counts[warp][digit] + rank[k];
+            if (last) {
+                keys_out[pos] = key[k];
+                values_out[pos] = val[k];
+            } else {
+                sm.keys[pos] = key[k];
+                sm.vals[pos] = val[k];
+            }
+        }
+        if (drop) {  // later passes (and the caller) see only the kept keys
+            n = static_cast<int>(all);
+            if (threadIdx.x == 0) *kept = n;
+            drop = false;
+        }
+        bit += digit_bits;
+        __syncthreads();
     }
 }
 
@@ -535,13 +671,20 @@ __global__ void __launch_bounds__(256) tile_ranges(const uint32_t* __restrict__ 
 
 // ---------------------------------------------------------------- host side
 // Words of the sort scratch for max_count pairs: four passes' digit totals
-// (kTotalCopies rows of 256 each), then one 256-bin histogram per 3072-key
-// block (the byte size adds 256 bytes of alignment slack).
+// (kTotalCopies rows of 256 each), then one 256-bin histogram per block
+// (the byte size adds 256 bytes of alignment slack).
 constexpr size_t kDigitTotalWords = static_cast<size_t>(kBins) * kTotalCopies;
+// Blocks of any sort of at most max_count pairs (a scratch made for max_count also
+// serves smaller sorts, whose blocks may be the smaller ones).
+constexpr size_t radix_sort_max_blocks(int max_count) {
+    const size_t n = static_cast<size_t>(max_count > 0 ? max_count : 1);
+    const size_t mid = (n < kMidCount ? n : kMidCount);
+    const size_t large = (n + kSortChunk - 1) / kSortChunk;
+    const size_t small = (mid + kSortThreads * kMidItems - 1) / (kSortThreads * kMidItems);
+    return large > small ? large : small;
+}
 constexpr size_t radix_sort_scratch_words(int max_count) {
-    return static_cast<size_t>(kBins) * ((static_cast<size_t>(max_count > 0 ? max_count : 1) + kSortChunk - 1) /
-                                         kSortChunk) +
-           kDigitTotalWords * 4;
+    return static_cast<size_t>(kBins) * radix_sort_max_blocks(max_count) + kDigitTotalWords * 4;
 }
 
 size_t radix_sort_scratch_bytes(int max_count) {
@@ -550,10 +693,43 @@ size_t radix_sort_scratch_bytes(int max_count) {
 
 RadixSortScratch radix_sort_scratch(void* base, int max_count) {
     RadixSortScratch s;
-    s.max_blocks = static_cast<size_t>(ceil_div(max_count > 0 ? max_count : 1, kSortChunk));
+    s.max_blocks = radix_sort_max_blocks(max_count);
     s.digit_total = static_cast<uint32_t*>(base);
     s.block_hist = s.digit_total + kDigitTotalWords * 4;
     return s;
+}
+
+// Raises the small sort's dynamic shared-memory limit, once per device.
+static int configure_small() {
+    static std::atomic<bool> configured[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return GSN_ERR_CUDA;
+    if (!configured[device].load()) {
+        if (cudaFuncSetAttribute(radix_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(SmallSmem))) != cudaSuccess)
+            return GSN_ERR_CUDA;
+        configured[device].store(true);
+    }
+    return GSN_OK;
+}
+
+// One pass of the general sort with kItems keys per thread.
+template <int kItems>
+static void radix_pass(uint32_t* kin, uint32_t* vin, uint32_t* kout, uint32_t* vout, bool identity, bool drop,
+                       const int* count, int max_count, int bit, int digit_bits, uint32_t* totals,
+                       const RadixSortScratch& scratch, cudaStream_t stream) {
+    const int blocks = ceil_div(max_count, kItems * kSortThreads);
+    const uint32_t mask = (1u << digit_bits) - 1u;
+    auto up = drop ? radix_upsweep<true, kItems> : radix_upsweep<false, kItems>;
+    launch_step(up, blocks, kSortThreads, 0, stream, kin, count, max_count, bit, mask, scratch.block_hist,
+                scratch.max_blocks, totals);
+    launch_step(radix_scan, 1 << digit_bits, kSortThreads, 0, stream, count, max_count, kItems * kSortThreads,
+                scratch.block_hist, scratch.max_blocks, totals);
+    auto down = identity ? (drop ? radix_downsweep<true, true, kItems> : radix_downsweep<true, false, kItems>)
+                         : (drop ? radix_downsweep<false, true, kItems> : radix_downsweep<false, false, kItems>);
+    const uint32_t* values = identity ? nullptr : vin;
+    launch_step(down, blocks, kSortThreads, 0, stream, kin, values, kout, vout, count, max_count, bit, mask,
+                digit_bits, scratch.block_hist, scratch.max_blocks);
 }
 
 static int radix_sort_impl(uint32_t* keys, uint32_t* values, uint32_t* keys_alt, uint32_t* values_alt,
@@ -564,9 +740,19 @@ static int radix_sort_impl(uint32_t* keys, uint32_t* values, uint32_t* keys_alt,
     if (max_count <= 0 || end_bit <= begin_bit) return GSN_OK;
     const int passes = (end_bit - begin_bit + 7) / 8;
     if (passes > 4 || !keys || !keys_alt || !values || !values_alt) return GSN_ERR_INVALID_ARGUMENT;
+    *result_in_alt = (passes % 2) == 1;
+    if (max_count <= kSmallCount) {
+        const int st = configure_small();
+        if (st != GSN_OK) return st;
+        // all inputs are read before the first output is written, so the pairs may be
+        // sorted in place
+        launch_step(radix_small, 1, kSmallThreads, sizeof(SmallSmem), stream, keys, values,
+                    *result_in_alt ? keys_alt : keys, *result_in_alt ? values_alt : values, count_device, max_count,
+                    begin_bit, end_bit, identity_values, kept_device);
+        return launched(1);
+    }
     if (cudaMemsetAsync(scratch.digit_total, 0, sizeof(uint32_t) * kDigitTotalWords * passes, stream) != cudaSuccess)
         return GSN_ERR_CUDA;
-    const int blocks = ceil_div(max_count, kSortChunk);
     uint32_t *kin = keys, *vin = values, *kout = keys_alt, *vout = values_alt;
     const int* count = count_device;
     // the key bits split into passes of near-equal width (13 tile bits: 7 + 6),
@@ -575,45 +761,23 @@ static int radix_sort_impl(uint32_t* keys, uint32_t* values, uint32_t* keys_alt,
     int bit = begin_bit;
     for (int p = 0; p < passes; ++p) {
         const int digit_bits = width / passes + (p < width % passes ? 1 : 0);
-        const uint32_t mask = (1u << digit_bits) - 1u;
-        const int bins = 1 << digit_bits;
-        uint32_t* dt = scratch.digit_total + kDigitTotalWords * p;
-        const bool drop = kept_device && p == 0;
-        if (drop)
-            launch_step(radix_upsweep<true>, blocks, kSortThreads, 0, stream, kin, count, max_count, bit, mask,
-                        scratch.block_hist, scratch.max_blocks, dt);
+        uint32_t* totals = scratch.digit_total + kDigitTotalWords * p;
+        const bool drop = kept_device && p == 0, identity = identity_values && p == 0;
+        if (max_count <= kMidCount)
+            radix_pass<kMidItems>(kin, vin, kout, vout, identity, drop, count, max_count, bit, digit_bits, totals,
+                                  scratch, stream);
         else
-            launch_step(radix_upsweep<false>, blocks, kSortThreads, 0, stream, kin, count, max_count, bit, mask,
-                        scratch.block_hist, scratch.max_blocks, dt);
-        launch_step(radix_scan, bins, kSortThreads, 0, stream, count, max_count, scratch.block_hist,
-                    scratch.max_blocks, dt);
-        const uint32_t* vsrc = identity_values && p == 0 ? nullptr : vin;
-        if (identity_values && p == 0 && drop)
-            launch_step(radix_downsweep<true, true>, blocks, kSortThreads, 0, stream,
-                kin, vsrc, kout, vout, count, max_count, bit, mask, digit_bits, scratch.block_hist,
-                scratch.max_blocks);
-        else if (identity_values && p == 0)
-            launch_step(radix_downsweep<true, false>, blocks, kSortThreads, 0, stream,
-                kin, vsrc, kout, vout, count, max_count, bit, mask, digit_bits, scratch.block_hist,
-                scratch.max_blocks);
-        else if (drop)
-            launch_step(radix_downsweep<false, true>, blocks, kSortThreads, 0, stream,
-                kin, vsrc, kout, vout, count, max_count, bit, mask, digit_bits, scratch.block_hist,
-                scratch.max_blocks);
-        else
-            launch_step(radix_downsweep<false, false>, blocks, kSortThreads, 0, stream,
-                kin, vsrc, kout, vout, count, max_count, bit, mask, digit_bits, scratch.block_hist,
-                scratch.max_blocks);
+            radix_pass<kSortItems>(kin, vin, kout, vout, identity, drop, count, max_count, bit, digit_bits, totals,
+                                   scratch, stream);
         if (drop) {
             // later passes (and the caller) see only the kept keys
-            launch_step(radix_kept, 1, kBins, 0, stream, dt, kept_device);
+            launch_step(radix_kept, 1, kBins, 0, stream, totals, kept_device);
             count = kept_device;
         }
         uint32_t* tk = kin; kin = kout; kout = tk;
         uint32_t* tv = vin; vin = vout; vout = tv;
         bit += digit_bits;
     }
-    *result_in_alt = (passes % 2) == 1;
     return launched(3 * passes + (kept_device ? 1 : 0));
 }
 
