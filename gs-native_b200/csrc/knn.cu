@@ -2,7 +2,7 @@
 //
 // Same result as ComputeMeanDist2Cuda (knn.cu:16-255): for every point the mean
 // of its (up to) three smallest squared distances to the other points, 0 when
-// there are fewer than two points. The structure is a linear BVH: 30-bit Morton
+// there are fewer than two points. The structure is a linear BVH: 30-bit Hilbert
 // codes over the bounding box, a stable radix sort (sort.cu), the points copied
 // into that order, buckets of 8 consecutive points as leaves and boxes of 32
 // children above them (three levels at 100k points, two launches to build).
@@ -12,9 +12,12 @@
 // neighbour closely, then walks the tree once for all of them: the 32 lanes test
 // a node's 32 child boxes against the warp's bounding box at once, the child on
 // the warp's own path is entered first, and a leaf's points are read once for 32
-// queries. A thread-per-point walk of a binary tree of the same leaves spent its
-// time on divergent, dependent loads (order, then point): the whole search took
-// 2,433 us at 100k points of a volume and two shells, and takes 345 us so.
+// queries. Along a Hilbert curve neighbours in order are neighbours in space; a Morton
+// order's jumps gave single warps boxes with 6,467 of the 12,500 leaves in reach (191
+// at most so), and those warps decided the time: a search of 100k points of a volume
+// and two shells took 377 us with it and takes 186 us. A thread-per-point walk of a
+// binary tree of the same leaves spent its time on divergent, dependent loads (order,
+// then point): 2,433 us.
 //
 // Squared distances are evaluated without contraction ((dx*dx + dy*dy) + dz*dz,
 // each rounded) and ties go to the smaller index, so the neighbour indices equal
@@ -112,23 +115,49 @@ __global__ void bounds_kernel(const float* __restrict__ pts, int n, unsigned int
     if (threadIdx.x < 6) atomicMin(bounds + threadIdx.x, s[threadIdx.x]);
 }
 
-__global__ void morton_kernel(const float* __restrict__ pts, int n, const unsigned int* __restrict__ bounds,
-                              uint32_t* __restrict__ keys) {
+// Position of a cell along the Hilbert curve of 2^10 cells per axis (J. Skilling,
+// "Programming the Hilbert curve", 2004: axes to transposed index).
+__device__ __forceinline__ uint32_t hilbert30(uint32_t x[3]) {
+#pragma unroll
+    for (uint32_t q = 1u << 9; q > 1u; q >>= 1) {
+        const uint32_t low = q - 1u;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (x[i] & q) {
+                x[0] ^= low;
+            } else {
+                const uint32_t t = (x[0] ^ x[i]) & low;
+                x[0] ^= t;
+                x[i] ^= t;
+            }
+        }
+    }
+    x[1] ^= x[0];
+    x[2] ^= x[1];
+    uint32_t t = 0;
+#pragma unroll
+    for (uint32_t q = 1u << 9; q > 1u; q >>= 1)
+        if (x[2] & q) t ^= q - 1u;
+    return (spread10(x[0] ^ t) << 2) | (spread10(x[1] ^ t) << 1) | spread10(x[2] ^ t);
+}
+
+__global__ void curve_kernel(const float* __restrict__ pts, int n, const unsigned int* __restrict__ bounds,
+                             uint32_t* __restrict__ keys) {
     pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    unsigned int c[3];
+    uint32_t c[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         float lo = ordered_to_float(bounds[a]), hi = ordered_to_float(~bounds[3 + a]);
         float ext = hi - lo;
         float t = ext > 0.0f ? (pts[3ll * i + a] - lo) / ext : 0.0f;
-        c[a] = static_cast<unsigned int>(fminf(fmaxf(t * 1023.0f, 0.0f), 1023.0f));
+        c[a] = static_cast<uint32_t>(fminf(fmaxf(t * 1023.0f, 0.0f), 1023.0f));
     }
-    keys[i] = spread10(c[0]) | (spread10(c[1]) << 1) | (spread10(c[2]) << 2);
+    keys[i] = hilbert30(c);
 }
 
-// The points in Morton order with their index as the fourth word, the leaf boxes
+// The points in curve order with their index as the fourth word, the leaf boxes
 // (8 points each) and the boxes of 32 leaves: one block covers 256 points, which
 // is one box of the level above the leaves.
 __global__ void __launch_bounds__(kThreads) leaves_kernel(const float* __restrict__ pts,
@@ -198,7 +227,7 @@ __global__ void __launch_bounds__(1024) levels_kernel(KnnTree tree, float4* lo, 
 // Squared distance of the box [plo, phi] (a point when equal) to a node's box.
 // Each difference, square and sum is monotonic under rounding, so the distance of
 // a box is never above that of a point inside it.
-__device__ __forceinline__ float box_distance(float3 plo, float3 phi, float4 lo, float4 hi) {
+__device__ __forceinline__ float box_distance(float3 plo, float3 phi, float3 lo, float3 hi) {
     const float x = fmaxf(fmaxf(lo.x - phi.x, plo.x - hi.x), 0.0f);
     const float y = fmaxf(fmaxf(lo.y - phi.y, plo.y - hi.y), 0.0f);
     const float z = fmaxf(fmaxf(lo.z - phi.z, plo.z - hi.z), 0.0f);
@@ -277,14 +306,20 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
     int level = tree.levels - 1, base = 0;
     uint32_t masks[kMaxLevels];
     int bases[kMaxLevels];
-    // children of `base`'s node at `level` whose box is within the warp's largest bound
+    // this lane's child of `base`'s node at `level`: its box stays in registers, so that
+    // testing a child against every lane's point is six shuffles and no load
+    float3 clo = make_float3(0.0f, 0.0f, 0.0f), chi = clo;
+    auto load_children = [&]() {
+        const int child = min(base + lane, tree.count[level] - 1);
+        const float4 l = lo[tree.offset[level] + child], h = hi[tree.offset[level] + child];
+        clo = make_float3(l.x, l.y, l.z);
+        chi = make_float3(h.x, h.y, h.z);
+    };
+    // the children whose box is within the warp's largest bound of the warp's box
     auto candidates = [&]() {
+        load_children();
         const float widest = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(bound, 0.0f))));
-        const int child = base + lane;
-        bool near = false;
-        if (child < tree.count[level])
-            near = box_distance(qlo, qhi, lo[tree.offset[level] + child], hi[tree.offset[level] + child]) <= widest;
-        return __ballot_sync(kAll, near);
+        return __ballot_sync(kAll, base + lane < tree.count[level] && box_distance(qlo, qhi, clo, chi) <= widest);
     };
     uint32_t mask = candidates();
     while (true) {
@@ -292,6 +327,7 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
             if (++level >= tree.levels) break;
             mask = masks[level];
             base = bases[level];
+            if (mask) load_children();
             continue;
         }
         // the child that holds this warp's own points first: its neighbours tighten the bounds
@@ -300,9 +336,9 @@ __global__ void __launch_bounds__(kQueryThreads) query_kernel(const float4* __re
         mask &= ~(1u << c);
         const int node = base + c;
         if (level == 0 && node / (32 / kBucket) == warp) continue;  // the warp's own points, already done
-        if (!__any_sync(kAll, box_distance(p, p, lo[tree.offset[level] + node], hi[tree.offset[level] + node]) <=
-                                  bound))
-            continue;
+        const float3 l = make_float3(__shfl_sync(kAll, clo.x, c), __shfl_sync(kAll, clo.y, c), __shfl_sync(kAll, clo.z, c));
+        const float3 h = make_float3(__shfl_sync(kAll, chi.x, c), __shfl_sync(kAll, chi.y, c), __shfl_sync(kAll, chi.z, c));
+        if (!__any_sync(kAll, box_distance(p, p, l, h) <= bound)) continue;
         if (level > 0) {
             masks[level] = mask;
             bases[level] = base;
@@ -381,7 +417,7 @@ int launch_knn3(const float* points, int n, float* mean_dist2, int* neighbors, v
     auto* hi = reinterpret_cast<float4*>(w + L.hi);
     if (cudaMemsetAsync(bounds, 0xFF, 6 * sizeof(unsigned int), s) != cudaSuccess) return GSN_ERR_CUDA;
     launch_step(bounds_kernel, grid_for(n), kThreads, 0, s, points, n, bounds);
-    launch_step(morton_kernel, grid_for(n), kThreads, 0, s, points, n, bounds, keys);
+    launch_step(curve_kernel, grid_for(n), kThreads, 0, s, points, n, bounds, keys);
     int launches = 2;
     bool alt = false;
     RadixSortScratch scratch = radix_sort_scratch(w + L.sort, n);
