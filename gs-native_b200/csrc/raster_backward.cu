@@ -37,8 +37,11 @@
 //     800 records, and the longest list decided the time;
 //   * a segment is a warp's whole work (a loop over segments made the compiler hold every
 //     pixel's inputs across it: 168 registers, or spills at 128, and 25 % more time).
+//   * the exact form skips the pairs of a quadrant that the record's ellipse does not
+//     reach (93 -> 67 us at 4,096 Gaussians and 128x128, neutral at 1.2M); in the fast
+//     form the branches cost more than the skipped arithmetic (468 -> 506 us at 3.0M).
 // Bound by instruction issue at 16 warps per SM (116 registers). Exact form at 1.2M
-// Gaussians and 1600x1064 602 -> 582 us, at 4,096 and 128x128 130 -> 93 us; fast form at
+// Gaussians and 1600x1064 602 -> 582 us, at 4,096 and 128x128 130 -> 67 us; fast form at
 // 3.0M and 2048x1360 487 -> 468 us, at 100k and 800x532 320 -> 260 us.
 // Per-Gaussian output (12 floats, Gaussian-major): d(u, v), d(cov a, b, c),
 // d(opacity logit), d(r, g, b), sum|du|, sum|dv|, 0.
@@ -54,7 +57,19 @@ namespace {
 constexpr int kVals = 12;
 constexpr int kFields = 11;     // values of a record that are not padding
 constexpr int kSumRow = 36;     // a value's 32 lanes, padded: rows 16 bytes apart in the banks
-constexpr int kPairs = 4;       // pixel pairs per lane: column px, rows y0 + 4h and y0 + 4h + 2
+constexpr int kPairs = 4;       // pixel pairs per lane
+
+// Where pair h of a lane lies in the tile. Exact form: one pair in each 8x8 quadrant,
+// so that a quadrant out of a record's reach is a pair to skip; fast form: four pairs
+// down one column, which share the column's terms.
+template <bool kFast>
+struct PairLayout {
+    static __device__ __forceinline__ int lane_x(int lane) { return kFast ? lane & 15 : lane & 7; }
+    static __device__ __forceinline__ int lane_y(int lane) { return kFast ? lane >> 4 : lane >> 3; }
+    static __device__ __forceinline__ constexpr int column(int h) { return kFast ? 0 : 8 * (h & 1); }
+    static __device__ __forceinline__ constexpr int row(int h) { return kFast ? 4 * h : 8 * (h >> 1); }
+    static constexpr int kStep = kFast ? 2 : 4;  // between the pair's two rows
+};
 constexpr int kBatch = 32;      // records staged per batch (one per lane)
 
 // Element-wise atomic add of four floats at a 16-byte aligned global address
@@ -86,9 +101,9 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     if (from >= bound) return;
     const int to = blockIdx.y + 1 == gridDim.y ? bound : min(bound, from + kSegment);
     const int tx = tile % a.cam.tile_count_x, ty = tile / a.cam.tile_count_x;
-    const int px = tx * kTile + (lane & 15);
-    const int y0 = ty * kTile + (lane >> 4);
-    const float fx = static_cast<float>(px), ny0 = -static_cast<float>(y0);
+    using Layout = PairLayout<kFast>;
+    const int x0 = tx * kTile + Layout::lane_x(lane), y0 = ty * kTile + Layout::lane_y(lane);
+    const float fx0 = static_cast<float>(x0), ny0 = -static_cast<float>(y0);
     for (int k = lane; k < kBatch; k += 32) s_acc[k * kVals + 11] = 0.0f;  // the padding slot
 
     // per pixel pair: T, P - S (P = dL/dcolour . colour in front of the
@@ -99,7 +114,7 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     if (from > 0) checkpoint = a.checkpoints + checkpoint_slot(begin, tile, from) * kTilePixels;
 #pragma unroll
     for (int p = 0; p < 2 * kPairs; ++p) {
-        const int py = y0 + 2 * p;
+        const int px = x0 + Layout::column(p >> 1), py = y0 + Layout::row(p >> 1) + Layout::kStep * (p & 1);
         float gi[3] = {0.0f, 0.0f, 0.0f};
         float S = 0.0f, T = 1.0f, P = 0.0f;
         limit[p] = 0;
@@ -112,7 +127,7 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
             }
             limit[p] = a.contributors[pix];
             if (checkpoint) {
-                const float4 state = checkpoint[(py - ty * kTile) * kTile + (lane & 15)];
+                const float4 state = checkpoint[(py - ty * kTile) * kTile + px - tx * kTile];
                 T = state.x;
                 P = gi[0] * state.y + gi[1] * state.z + gi[2] * state.w;
             }
@@ -132,9 +147,9 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     }
     for (int rel = from; rel < to; rel += kBatch) {
         const int batch = min(kBatch, to - rel);
-        // stage one record per lane; the take flags (a record some pixel of the
-        // tile took in the forward pass) become a ballot
-        bool flag = false;
+        // stage one record per lane; the quadrants that a record some pixel of the tile
+        // took in the forward pass can reach become four ballots (the fast form: all four)
+        bool flag[kPairs] = {};
         if (lane < batch) {
             const int64_t r = begin + rel + lane;
             const uint32_t id = __ldg(a.tile_ids + r);
@@ -146,9 +161,20 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
             const float* c = reinterpret_cast<const float*>(a.colors) + 3ull * id;
             s_color[lane] = make_float3(__ldg(c), __ldg(c + 1), __ldg(c + 2));
             s_aux[lane] = kFast ? fast_record(q) : make_float4(alpha_floor(q.w), 0.0f, 0.0f, 0.0f);
-            flag = ((a.record_warps[r >> 5] | a.record_warps[a.record_words + (r >> 5)]) >> (r & 31)) & 1u;
+            if (((a.record_warps[r >> 5] | a.record_warps[a.record_words + (r >> 5)]) >> (r & 31)) & 1u) {
+                const float limit_q = cull_limit(mean, q);
+#pragma unroll
+                for (int h = 0; h < kPairs; ++h) {
+                    const float qx = static_cast<float>(tx * kTile + 8 * (h & 1));
+                    const float qy = static_cast<float>(ty * kTile + 8 * (h >> 1));
+                    flag[h] = kFast || region_hit(mean, q.x, 2.0f * q.y, q.z, limit_q, qx, qx + 7.0f, qy, qy + 7.0f);
+                }
+            }
         }
-        uint32_t m = __ballot_sync(0xffffffffu, flag);
+        uint32_t reach[kPairs];
+#pragma unroll
+        for (int h = 0; h < kPairs; ++h) reach[h] = __ballot_sync(0xffffffffu, flag[h]);
+        uint32_t m = (reach[0] | reach[1]) | (reach[2] | reach[3]);
         const uint32_t taken = m;
         __syncwarp();
         int parity = 0, previous = 0;
@@ -161,10 +187,6 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
             const float4 q = s_conic[j];
             const float3 col = s_color[j];
             const float4 aux = s_aux[j];
-            const float dx = mu.x - fx;
-            const float qxdx = q.x * dx, qydx = q.y * dx;
-            const float Ax = fmaf(aux.x * dx, dx, aux.w), Bx = aux.y * dx;  // fast form
-            const Power power(q, dx);                                // exact form
             const float2 m1 = pk(-1.0f), one = pk(1.0f);
             float2 acc[9];
 #pragma unroll
@@ -172,17 +194,23 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
             float abs_u = 0.0f, abs_v = 0.0f;
 #pragma unroll
             for (int h = 0; h < kPairs; ++h) {
+                if (!kFast && !(reach[h] & bit)) continue;  // the same for every lane
+                const float dx = mu.x - (fx0 + static_cast<float>(Layout::column(h)));
+                const float qxdx = q.x * dx, qydx = q.y * dx;
                 // -y of the pair's pixels, exact in fp32
-                const float2 ny = add2(pk(ny0), make_float2(-4.0f * h, -4.0f * h - 2.0f));
+                const float2 ny = add2(pk(ny0), make_float2(-static_cast<float>(Layout::row(h)),
+                                                            -static_cast<float>(Layout::row(h) + Layout::kStep)));
                 const float2 dy = add2(pk(mu.y), ny);
                 float2 alpha;
                 if constexpr (kFast) {
+                    const float Ax = fmaf(aux.x * dx, dx, aux.w), Bx = aux.y * dx;
                     const float2 pw2 = fma2(fma2(pk(aux.z), dy, pk(Bx)), dy, pk(Ax));
                     const bool take0 = idx < limit[2 * h] && pw2.x >= kLog2AlphaMin;
                     const bool take1 = idx < limit[2 * h + 1] && pw2.y >= kLog2AlphaMin;
                     alpha.x = take0 ? fminf(kAlphaMax, ex2_approx(pw2.x)) : 0.0f;
                     alpha.y = take1 ? fminf(kAlphaMax, ex2_approx(pw2.y)) : 0.0f;
                 } else {
+                    const Power power(q, dx);
                     const float pw0 = power.at(dy.x), pw1 = power.at(dy.y);
                     const float raw0 = gaussian_weight<false>(q.w, pw0);
                     const float raw1 = gaussian_weight<false>(q.w, pw1);
