@@ -7,16 +7,18 @@
 //
 // Both passes are bound by FP32 FMA issue (15,104 multiply-adds per trained
 // sample, 5,376 per inferred one), so they run as register-tiled GEMMs: a CTA of
-// 256 threads takes tiles of 64 samples, keeps the activations of a tile
+// 256 threads takes tiles of 128 samples, keeps the activations of a tile
 // feature-major in shared memory and the weights (widened to fp32 once per CTA)
-// beside them, and every thread forms a 4 x 4 block of a layer's outputs, two
-// 16-byte shared loads per 16 FMAs. CTAs are persistent, two to three per SM; a
+// beside them, and every thread forms an 8 x 4 block of a layer's outputs: three
+// 16-byte shared loads per 32 FMAs, two of them the same for the whole warp. (4 x 4
+// blocks, two loads per 16 FMAs, were bound by shared memory: 294 us per fit step and
+// 119 us per inference of 300k samples against 277 and 98.) CTAs are persistent; a
 // training CTA holds its share of the weight gradients in registers over all of
 // its tiles and adds them to the global fp32 gradient once, in 16-byte vector
-// reductions. One thread per sample with its vectors in shared memory (two shared
-// loads and a widening per FMA, 5,508 atomics per 128 samples) took 1,620 us per
-// fit step and 149 us per inference of 300k samples; four steps and an inference
-// went from 7,029 to 1,311 us (FP32 FMA floor 0.53 ms).
+// reductions; the next tile's inputs are loaded while a tile is computed. One thread
+// per sample with its vectors in shared memory (two shared loads and a widening per
+// FMA, 5,508 atomics per 128 samples) took 1,620 and 149 us; four fit steps and an
+// inference went from 7,029 to 1,208 us (FP32 FMA floor 0.53 ms).
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -32,7 +34,7 @@ constexpr int kOffW3 = kOffB2 + kHid, kOffB3 = kOffW3 + kOut * kHid;
 static_assert(kOffB3 + kOut == kMlpParams, "weight layout");
 
 constexpr int kMlpThreads = 256;
-constexpr int kSampleTile = 64;        // samples per tile
+constexpr int kSampleTile = 128;       // samples per tile
 constexpr int kRow = kSampleTile + 4;  // padded row: rows 16 bytes apart in the banks
 constexpr int kW3Row = kHid + 4;
 
@@ -57,37 +59,39 @@ __device__ __forceinline__ void load_weights(const __half* __restrict__ src, Wei
     }
 }
 
-// This thread's 4 x 4 block: rows row0 .. row0 + 3 of a layer, samples col0 ..
-// col0 + 3. A warp covers 16 rows x 32 samples, so its two 16-byte loads per step
-// read 64 and 128 distinct bytes.
+// This thread's 8 x 4 block: rows row0 .. row0 + 7 of a layer (the same for a warp),
+// samples col0 .. col0 + 3.
+constexpr int kBlockRows = 8;
+
 struct Block {
     int row0, col0;
     __device__ __forceinline__ Block() {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        row0 = 4 * ((lane >> 3) + 4 * (warp >> 1));
-        col0 = 4 * ((lane & 7) + 8 * (warp & 1));
+        row0 = kBlockRows * (threadIdx.x >> 5);
+        col0 = 4 * (threadIdx.x & 31);
     }
 };
+static_assert(kBlockRows * (kMlpThreads / 32) == kHid && 4 * 32 == kSampleTile, "one block per thread");
 
 // acc[i][j] += sum over k of w[k][row0 + i] * x[k][col0 + j], k ascending.
 template <int K>
 __device__ __forceinline__ void block_product(const float* __restrict__ w, const float* __restrict__ x, const Block& b,
-                                              float acc[4][4]) {
-#pragma unroll 8
+                                              float acc[kBlockRows][4]) {
+#pragma unroll 4
     for (int k = 0; k < K; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(w + k * kHid + b.row0);
+        const float4 a0 = *reinterpret_cast<const float4*>(w + k * kHid + b.row0);
+        const float4 a1 = *reinterpret_cast<const float4*>(w + k * kHid + b.row0 + 4);
         const float4 v = *reinterpret_cast<const float4*>(x + k * kRow + b.col0);
-        const float ai[4] = {a.x, a.y, a.z, a.w}, vj[4] = {v.x, v.y, v.z, v.w};
+        const float ai[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, vj[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < kBlockRows; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ai[i], vj[j], acc[i][j]);
     }
 }
 
-__device__ __forceinline__ void store_rows(float* dst, const Block& b, const float v[4][4]) {
+__device__ __forceinline__ void store_rows(float* dst, const Block& b, const float v[kBlockRows][4]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < kBlockRows; ++i)
         *reinterpret_cast<float4*>(dst + (b.row0 + i) * kRow + b.col0) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
 }
 
@@ -95,39 +99,49 @@ __device__ __forceinline__ void store_rows(float* dst, const Block& b, const flo
 // block, into h.
 template <int K>
 __device__ __forceinline__ void layer(const float* w, const float* bias, const float* x, const Block& b, float* out,
-                                      float h[4][4]) {
+                                      float h[kBlockRows][4]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < kBlockRows; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) h[i][j] = bias[b.row0 + i];
     block_product<K>(w, x, b, h);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < kBlockRows; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) h[i][j] = fmaxf(h[i][j], 0.0f);
     store_rows(out, b, h);
 }
 
-// The tile's features, feature-major (zeros past n).
-__device__ __forceinline__ void load_tile(const float* __restrict__ features, int64_t first, int n, float* f) {
+// A tile's features on their way to shared memory (zeros past n): loaded ahead of the
+// tile's turn, stored feature-major at it.
+struct TileFeatures {
+    static constexpr int kPer = kSampleTile * kIn / kMlpThreads;
+    float v[kPer];
+    __device__ __forceinline__ void load(const float* __restrict__ features, int64_t first, int n) {
 #pragma unroll
-    for (int u = 0; u < kSampleTile * kIn / kMlpThreads; ++u) {
-        const int i = threadIdx.x + u * kMlpThreads;
-        const int s = i / kIn, k = i % kIn;
-        f[k * kRow + s] = first + s < n ? features[(first + s) * kIn + k] : 0.0f;
+        for (int u = 0; u < kPer; ++u) {
+            const int i = threadIdx.x + u * kMlpThreads;
+            v[u] = first + i / kIn < n ? features[first * kIn + i] : 0.0f;
+        }
     }
-}
-
-// The four logits of this thread's sample: thread t has output a = t & 3 of sample
-// t >> 2. Two neighbouring samples' products are formed by the eight threads of the
-// pair, each over half of the inputs.
-__device__ __forceinline__ void tile_logits(const Weights& w, const float* __restrict__ h2, float logit[kOut]) {
-    const int a = threadIdx.x & 3, half = (threadIdx.x >> 2) & 1, pair = threadIdx.x >> 3;
-    float p0 = half ? 0.0f : w.b3[a], p1 = p0;
-    const float* wr = w.w3 + a * kW3Row + half * (kHid / 2);
-    const float* hr = h2 + half * (kHid / 2) * kRow + 2 * pair;
+    __device__ __forceinline__ void store(float* f) const {
 #pragma unroll
-    for (int o = 0; o < kHid / 2; o += 4) {
+        for (int u = 0; u < kPer; ++u) {
+            const int i = threadIdx.x + u * kMlpThreads;
+            f[(i % kIn) * kRow + i / kIn] = v[u];
+        }
+    }
+};
+
+// Output a = t & 3 of the two samples 2 (t >> 2) and 2 (t >> 2) + 1, then all four
+// outputs of both by the quad of threads that shares them.
+__device__ __forceinline__ void tile_logits(const Weights& w, const float* __restrict__ h2, float logit[2][kOut]) {
+    const int a = threadIdx.x & 3;
+    float p0 = w.b3[a], p1 = p0;
+    const float* wr = w.w3 + a * kW3Row;
+    const float* hr = h2 + 2 * (threadIdx.x >> 2);
+#pragma unroll 4
+    for (int o = 0; o < kHid; o += 4) {
         const float4 q = *reinterpret_cast<const float4*>(wr + o);
         const float qi[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -137,12 +151,16 @@ __device__ __forceinline__ void tile_logits(const Weights& w, const float* __res
             p1 = fmaf(qi[i], v.y, p1);
         }
     }
-    p0 += __shfl_xor_sync(0xffffffffu, p0, 4);
-    p1 += __shfl_xor_sync(0xffffffffu, p1, 4);
-    const float mine = half ? p1 : p0;
     const int quad = threadIdx.x & 28;
 #pragma unroll
-    for (int q = 0; q < kOut; ++q) logit[q] = __shfl_sync(0xffffffffu, mine, quad | q);
+    for (int q = 0; q < kOut; ++q) {
+        logit[0][q] = __shfl_sync(0xffffffffu, p0, quad | q);
+        logit[1][q] = __shfl_sync(0xffffffffu, p1, quad | q);
+    }
+}
+
+__device__ __forceinline__ float pick(const float v[kOut], int a) {
+    return a == 0 ? v[0] : a == 1 ? v[1] : a == 2 ? v[2] : v[3];
 }
 
 struct InferSmem {
@@ -150,7 +168,7 @@ struct InferSmem {
     float f[kIn * kRow], h1[kHid * kRow], h2[kHid * kRow];
 };
 
-__global__ void __launch_bounds__(kMlpThreads, 3) mlp_infer_kernel(const float* __restrict__ features, int n,
+__global__ void __launch_bounds__(kMlpThreads, 2) mlp_infer_kernel(const float* __restrict__ features, int n,
                                                                    const __half* __restrict__ weights,
                                                                    float confidence, int8_t* __restrict__ actions,
                                                                    float* __restrict__ probs) {
@@ -159,39 +177,44 @@ __global__ void __launch_bounds__(kMlpThreads, 3) mlp_infer_kernel(const float* 
     load_weights(weights, m.w);
     const Block block;
     const int tiles = ceil_div(n, kSampleTile);
+    TileFeatures next;
+    next.load(features, static_cast<int64_t>(blockIdx.x) * kSampleTile, n);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t first = static_cast<int64_t>(tile) * kSampleTile;
         __syncthreads();  // the weights, or the previous tile's readers
-        load_tile(features, first, n, m.f);
+        next.store(m.f);
         __syncthreads();
-        float h[4][4];
+        next.load(features, first + static_cast<int64_t>(gridDim.x) * kSampleTile, n);
+        float h[kBlockRows][4];
         layer<kIn>(m.w.w1, m.w.b1, m.f, block, m.h1, h);
         __syncthreads();
         layer<kHid>(m.w.w2, m.w.b2, m.h1, block, m.h2, h);
         __syncthreads();
-        float logit[kOut];
+        float logit[2][kOut];
         tile_logits(m.w, m.h2, logit);
-        float mx = logit[0];
-        int best = 0;
-#pragma unroll
-        for (int a = 1; a < kOut; ++a)
-            if (logit[a] > mx) {
-                mx = logit[a];
-                best = a;
-            }
-        float e[kOut], sum = 0.0f;
-#pragma unroll
-        for (int a = 0; a < kOut; ++a) {
-            e[a] = __expf(logit[a] - mx);
-            sum += e[a];
-        }
-        const int64_t id = first + (threadIdx.x >> 2);
         const int a = threadIdx.x & 3;
-        if (id >= n) continue;
-        const float mine = a == 0 ? e[0] : a == 1 ? e[1] : a == 2 ? e[2] : e[3];
-        if (probs) probs[id * kOut + a] = mine / sum;
-        const float top = best == 0 ? e[0] : best == 1 ? e[1] : best == 2 ? e[2] : e[3];
-        if (a == 0) actions[id] = top / sum >= confidence ? static_cast<int8_t>(best) : static_cast<int8_t>(-1);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float mx = logit[half][0];
+            int best = 0;
+#pragma unroll
+            for (int q = 1; q < kOut; ++q)
+                if (logit[half][q] > mx) {
+                    mx = logit[half][q];
+                    best = q;
+                }
+            float e[kOut], sum = 0.0f;
+#pragma unroll
+            for (int q = 0; q < kOut; ++q) {
+                e[q] = __expf(logit[half][q] - mx);
+                sum += e[q];
+            }
+            const int64_t id = first + 2 * (threadIdx.x >> 2) + half;
+            if (id >= n) continue;
+            if (probs) probs[id * kOut + a] = pick(e, a) / sum;
+            if (a == half)
+                actions[id] = pick(e, best) / sum >= confidence ? static_cast<int8_t>(best) : static_cast<int8_t>(-1);
+        }
     }
 }
 
@@ -211,27 +234,27 @@ struct TrainSmem {
 };
 static_assert(kMlpParams % 4 == 0 && kMlpParams <= 2 * kHid * kRow, "the gradient leaves in 16-byte vectors over h1, h2");
 
-// sum over the tile of x[i][s] * y[j][s] added to acc[i][j], rows row + 16 i of x and
-// col + 16 j of y.
+// sum over samples first .. first + 31 of x[i][s] * y[j][s] added to acc[i][j], rows
+// row + 8 i of x and col + 8 j of y.
 template <int I, int J>
 __device__ __forceinline__ void outer_product(const float* __restrict__ x, const float* __restrict__ y, int row,
-                                              int col, float acc[I][J]) {
-#pragma unroll 2
-    for (int s = 0; s < kSampleTile; s += 4) {
-        float4 a[I], b[J];
+                                              int col, int first, float acc[I][J]) {
+#pragma unroll 1
+    for (int s = first; s < first + 32; s += 4) {
+        float4 a[I];
 #pragma unroll
-        for (int i = 0; i < I; ++i) a[i] = *reinterpret_cast<const float4*>(x + (row + 16 * i) * kRow + s);
+        for (int i = 0; i < I; ++i) a[i] = *reinterpret_cast<const float4*>(x + (row + 8 * i) * kRow + s);
 #pragma unroll
-        for (int j = 0; j < J; ++j) b[j] = *reinterpret_cast<const float4*>(y + (col + 16 * j) * kRow + s);
+        for (int j = 0; j < J; ++j) {
+            const float4 b = *reinterpret_cast<const float4*>(y + (col + 8 * j) * kRow + s);
 #pragma unroll
-        for (int i = 0; i < I; ++i)
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-                acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-                acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-                acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+            for (int i = 0; i < I; ++i) {
+                acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+                acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+                acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+                acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
             }
+        }
     }
 }
 
@@ -248,7 +271,7 @@ __device__ __forceinline__ float row_sum(const float* __restrict__ row) {
     return v;
 }
 
-__global__ void __launch_bounds__(kMlpThreads, 2) mlp_train_kernel(const float* __restrict__ features,
+__global__ void __launch_bounds__(kMlpThreads, 1) mlp_train_kernel(const float* __restrict__ features,
                                                                    const int* __restrict__ labels,
                                                                    const float* __restrict__ sample_weights, int n,
                                                                    float weight_norm,
@@ -261,59 +284,78 @@ __global__ void __launch_bounds__(kMlpThreads, 2) mlp_train_kernel(const float* 
     for (int i = threadIdx.x; i < kHid * kHid; i += kMlpThreads) m.w2_out[i] = __half2float(weights[kOffW2 + i]);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const Block block;
-    // weight gradients: rows ty + 16 i, inputs tx + 16 j of W2; inputs tx of W1
-    const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);
-    float d2[4][4] = {}, d1[4][1] = {}, d3 = 0.0f, db = 0.0f;
+    // weight gradients: two warps form all of them over a quarter of the tile's samples,
+    // a thread rows ty + 8 i and inputs tx + 8 j
+    const int tx = t & 7, ty = (t >> 3) & 7, part = t >> 6;
+    float d2[8][8] = {}, d1[8][2] = {}, d3 = 0.0f, db = 0.0f;
     double loss_sum = 0.0;
     const int tiles = ceil_div(n, kSampleTile);
+    const int a = t & 3;
+    // the inputs of the coming tile: features, and labels and weights of the two
+    // samples 2 (t >> 2) and 2 (t >> 2) + 1
+    TileFeatures next;
+    int next_label[2];
+    float next_weight[2];
+    auto load_next = [&](int64_t first) {
+        next.load(features, first, n);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int64_t id = first + 2 * (t >> 2) + half;
+            next_label[half] = id < n ? labels[id] : 0;
+            next_weight[half] = id < n ? sample_weights[id] * weight_norm : 0.0f;
+        }
+    };
+    load_next(static_cast<int64_t>(blockIdx.x) * kSampleTile);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t first = static_cast<int64_t>(tile) * kSampleTile;
         __syncthreads();  // the weights, or the previous tile's readers
-        load_tile(features, first, n, m.f);
-        const int64_t id = first + (t >> 2);
-        const bool live = id < n;
-        const int label = live ? labels[id] : 0;
-        const float sw = live ? sample_weights[id] * weight_norm : 0.0f;
+        next.store(m.f);
+        const int label[2] = {next_label[0], next_label[1]};
+        const float sw[2] = {next_weight[0], next_weight[1]};
         __syncthreads();
-        float h[4][4];
+        load_next(first + static_cast<int64_t>(gridDim.x) * kSampleTile);
+        float h[kBlockRows][4];
         layer<kIn>(m.w.w1, m.w.b1, m.f, block, m.h1, h);
         __syncthreads();
         layer<kHid>(m.w.w2, m.w.b2, m.h1, block, m.h2, h);
         __syncthreads();
         {   // softmax cross-entropy, weighted and normalised by the batch weight
-            float logit[kOut];
+            float logit[2][kOut], dl[2];
             tile_logits(m.w, m.h2, logit);
-            const float mx = fmaxf(fmaxf(logit[0], logit[1]), fmaxf(logit[2], logit[3]));
-            float e[kOut], sum = 0.0f;
 #pragma unroll
-            for (int a = 0; a < kOut; ++a) {
-                e[a] = expf(logit[a] - mx);
-                sum += e[a];
+            for (int half = 0; half < 2; ++half) {
+                const float mx = fmaxf(fmaxf(logit[half][0], logit[half][1]), fmaxf(logit[half][2], logit[half][3]));
+                float e[kOut], sum = 0.0f;
+#pragma unroll
+                for (int q = 0; q < kOut; ++q) {
+                    e[q] = expf(logit[half][q] - mx);
+                    sum += e[q];
+                }
+                dl[half] = sw[half] * (pick(e, a) / sum - (a == label[half] ? 1.0f : 0.0f));
+                if (loss && a == half && first + 2 * (t >> 2) + half < n) {
+                    const double lp =
+                        static_cast<double>(pick(logit[half], label[half]) - mx) - log(static_cast<double>(sum));
+                    loss_sum -= static_cast<double>(sw[half]) * lp;
+                }
             }
-            const int a = t & 3;
-            const float mine = a == 0 ? e[0] : a == 1 ? e[1] : a == 2 ? e[2] : e[3];
-            m.dl[a * kRow + (t >> 2)] = sw * (mine / sum - (a == label ? 1.0f : 0.0f));
-            if (live && loss && a == 0) {
-                const float own = label == 0 ? logit[0] : label == 1 ? logit[1] : label == 2 ? logit[2] : logit[3];
-                const double lp = static_cast<double>(own - mx) - log(static_cast<double>(sum));
-                loss_sum -= static_cast<double>(sw) * lp;
-            }
+            *reinterpret_cast<float2*>(m.dl + a * kRow + 2 * (t >> 2)) = make_float2(dl[0], dl[1]);
         }
         __syncthreads();
         {   // back through layer 3 and the second ReLU; the gradient of W3
-            float z[4][4] = {};
+            float z[kBlockRows][4] = {};
 #pragma unroll
-            for (int a = 0; a < kOut; ++a) {
-                const float4 q = *reinterpret_cast<const float4*>(m.w.w3 + a * kW3Row + block.row0);
-                const float4 v = *reinterpret_cast<const float4*>(m.dl + a * kRow + block.col0);
-                const float qi[4] = {q.x, q.y, q.z, q.w}, vj[4] = {v.x, v.y, v.z, v.w};
+            for (int q = 0; q < kOut; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(m.dl + q * kRow + block.col0);
+                const float vj[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < kBlockRows; ++i) {
+                    const float wq = m.w.w3[q * kW3Row + block.row0 + i];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) z[i][j] = fmaf(qi[i], vj[j], z[i][j]);
+                    for (int j = 0; j < 4; ++j) z[i][j] = fmaf(wq, vj[j], z[i][j]);
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < kBlockRows; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) z[i][j] = h[i][j] > 0.0f ? z[i][j] : 0.0f;
             store_rows(m.z2, block, z);
@@ -331,10 +373,10 @@ __global__ void __launch_bounds__(kMlpThreads, 2) mlp_train_kernel(const float* 
         }
         __syncthreads();
         {   // back through layer 2 and the first ReLU (into h2's place); the gradient of W2
-            float z[4][4] = {};
+            float z[kBlockRows][4] = {};
             block_product<kHid>(m.w2_out, m.z2, block, z);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < kBlockRows; ++i) {
                 const float4 v = *reinterpret_cast<const float4*>(m.h1 + (block.row0 + i) * kRow + block.col0);
                 z[i][0] = v.x > 0.0f ? z[i][0] : 0.0f;
                 z[i][1] = v.y > 0.0f ? z[i][1] : 0.0f;
@@ -342,23 +384,36 @@ __global__ void __launch_bounds__(kMlpThreads, 2) mlp_train_kernel(const float* 
                 z[i][3] = v.w > 0.0f ? z[i][3] : 0.0f;
             }
             store_rows(m.h2, block, z);
-            outer_product<4, 4>(m.z2, m.h1, ty, tx, d2);
+            outer_product<8, 8>(m.z2, m.h1, ty, tx, 32 * part, d2);
         }
         __syncthreads();
         // the gradients of W1 and of the biases (b1, b2, b3 by threads 0, 64, 128 on)
-        outer_product<4, 1>(m.h2, m.f, ty, tx, d1);
+        outer_product<8, 2>(m.h2, m.f, ty, tx, 32 * part, d1);
         if (t < 64) db += row_sum(m.h2 + t * kRow);
         else if (t < 128) db += row_sum(m.z2 + (t - 64) * kRow);
         else if (t < 128 + kOut) db += row_sum(m.dl + (t - 128) * kRow);
     }
     __syncthreads();
-    // the CTA's gradient in its flat layout over h1 and h2, then one vector reduction each
+    // the CTA's gradient in its flat layout over h1 and h2 (the four parts in turn),
+    // then one vector reduction each
     float* g = m.h1;
+    for (int turn = 0; turn < 4; ++turn) {
+        if (part == turn) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        g[kOffW1 + (ty + 16 * i) * kIn + tx] = d1[i][0];
+            for (int i = 0; i < 8; ++i) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) g[kOffW2 + (ty + 16 * i) * kHid + tx + 16 * j] = d2[i][j];
+                for (int j = 0; j < 2; ++j) {
+                    float* at = g + kOffW1 + (ty + 8 * i) * kIn + tx + 8 * j;
+                    *at = turn ? *at + d1[i][j] : d1[i][j];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float* at = g + kOffW2 + (ty + 8 * i) * kHid + tx + 8 * j;
+                    *at = turn ? *at + d2[i][j] : d2[i][j];
+                }
+            }
+        }
+        __syncthreads();
     }
     g[kOffW3 + t] = d3;
     if (t < 64) g[kOffB1 + t] = db;

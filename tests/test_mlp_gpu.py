@@ -43,9 +43,9 @@ def test_gpu_gradients_match_fp64_oracle():
     assert np.max(np.abs(g - gref)) <= 1e-4 * np.max(np.abs(gref)) + 1e-7
 
 
-@pytest.mark.parametrize("n", [1, 63, 64, 65, 2000, 40001])
+@pytest.mark.parametrize("n", [1, 63, 127, 128, 129, 2000, 40001])
 def test_ragged_tiles_match_the_fp64_oracle(n):
-    """Sizes around the 64-sample tile, one tile, fewer tiles than CTAs and several
+    """Sizes around the 128-sample tile, one tile, fewer tiles than CTAs and several
     per CTA: gradients as above, probabilities and confident actions of the inference."""
     f, labels, w = samples(n, n)
     mlp = gsn.Mlp(seed=n)
