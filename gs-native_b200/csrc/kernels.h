@@ -56,6 +56,7 @@ struct ProjectOutputs {
     uint32_t* depth_keys;    // [N] float bits of z, 0xFFFFFFFF when culled
     float* radii;            // [N] optional 3-sigma pixel radius (0 = culled), may be null
     int* cull_counts;        // [N] optional exact-culling record counts (16 x 16 tiles only), may be null
+    uint4* cull_spans;       // [N] with cull_counts: the kept column intervals (project.cu cull_count)
     int depth_key_shift;     // depth key = float bits >> shift (0: exact order; 8: 24-bit keys, fast forms)
 };
 // cam_dev (optional): device camera read instead of `cam` (batched form).
@@ -114,9 +115,15 @@ int launch_exclusive_scan(const int* in, const uint32_t* gather, int* out, int n
 // Emit one (tile, gaussian id) record per tile of every visible Gaussian, in
 // depth order. record_start[p] is the exclusive scan of tile counts in sorted
 // order; records beyond `capacity` are not written and set *overflow.
-int launch_emit_records(const uint32_t* sorted_ids, const int* record_start, const int4* rects,
-                        int n, int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids,
+// visible (optional, device): only the first *visible entries of the order exist.
+int launch_emit_records(const uint32_t* sorted_ids, const int* record_start, const int4* rects, int n,
+                        const int* visible, int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids,
                         int64_t capacity, int* overflow, cudaStream_t stream);
+
+// Both emitters run resident blocks over the visible Gaussians (the host does not know
+// their number): at most kEmitBlocks of 256 threads.
+constexpr int kEmitBlocks = 148 * 8;
+int emit_blocks(int lanes, int n);
 
 // Exact tile culling (project.cu): with ProjectOutputs::cull_counts set, the
 // projection also counts, per Gaussian, the tiles of its rect whose pixel
@@ -124,10 +131,10 @@ int launch_emit_records(const uint32_t* sorted_ids, const int* record_start, con
 // emits exactly those records in depth order. Dropped records are ones the blend
 // kernels skip at every pixel, so images and gradients are unchanged. A count
 // the emitter cannot reproduce sets *overflow to 2 (never expected).
-int launch_emit_records_culled(const uint32_t* sorted_ids, const int* record_start, const int4* rects,
-                               const float2* means, const float4* conic_opacity, int n, int tile_count_x,
-                               uint32_t* tile_keys, uint32_t* record_ids, int64_t capacity, int* overflow,
-                               cudaStream_t stream);
+int launch_emit_records_culled(const uint32_t* sorted_ids, const int* record_start, const uint4* cull_spans,
+                               const int4* rects, const float2* means, const float4* conic_opacity, int n,
+                               const int* visible, int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids,
+                               int64_t capacity, int* overflow, cudaStream_t stream);
 
 // Per-tile [begin, end) offsets of sorted tile keys (empty tiles included).
 int launch_tile_ranges(const uint32_t* sorted_tiles, const int* record_count_device, int max_records,

@@ -53,9 +53,13 @@ __device__ __forceinline__ void sh_basis(float x, float y, float z, float b[16])
 //
 // Per tile row the reachable columns form one interval: the ellipse's x-extent
 // inside the band of the row's pixel centres, found at the band edge nearest to
-// the ellipse's leftmost / rightmost point. Both functions are kept out of line
-// so that the counting (projection) and the emitting kernel run one and the same
-// instruction sequence on the same stored values and agree on every count.
+// the ellipse's leftmost / rightmost point. The projection finds the intervals and
+// keeps them for the emitter (a byte per row: 4 bits offset, 4 bits width) where the
+// rectangle has at most 8 rows and 15 columns, which all but a few Gaussians' have.
+// For the others the emitter finds them again: then both run the same functions kept
+// out of line, one and the same instruction sequence on the same stored values, and
+// agree on every count. The kept form takes the hardware's approximate square roots
+// and divides (a relative 1e-6 against paddings of 1e-3).
 struct CullShape {
     float mx, my;      // mean
     float B, inv_a;    // conic B, 1 / A
@@ -65,8 +69,22 @@ struct CullShape {
     int mode;          // 0: reaches no pixel, 1: keep whole rows, 2: ellipse spans
 };
 
-__device__ __noinline__ CullShape cull_shape(float2 mean, float4 q) {
-    CullShape s;
+template <bool kApprox>
+__device__ __forceinline__ float cull_sqrt(float x) {
+    if (!kApprox) return sqrtf(x);
+    float y;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <bool kApprox>
+__device__ __forceinline__ float cull_divide(float a, float b) {
+    return kApprox ? __fdividef(a, b) : a / b;
+}
+
+template <bool kApprox>
+__device__ __forceinline__ CullShape make_cull_shape(float2 mean, float4 q) {
+    CullShape s{};
     s.mode = 0;
     s.mx = mean.x;
     s.my = mean.y;
@@ -76,31 +94,33 @@ __device__ __noinline__ CullShape cull_shape(float2 mean, float4 q) {
     s.mode = 1;
     const float det = q.x * q.z - q.y * q.y;
     const float tr = 0.5f * (q.x + q.z);
-    const float disc = sqrtf(fmaxf(tr * tr - det, 0.0f));
-    const float kappa = (tr + disc) / fmaxf(tr - disc, 1e-30f);
+    const float disc = cull_sqrt<kApprox>(fmaxf(tr * tr - det, 0.0f));
+    const float kappa = cull_divide<kApprox>(tr + disc, fmaxf(tr - disc, 1e-30f));
     if (!(det > 0.0f) || !(kappa < 1e5f) || !isfinite(mean.x) || !isfinite(mean.y) || !isfinite(lo)) return s;
     const float Q = 2.0f * __logf(lo) * (1.02f + 1e-6f * kappa) + 0.05f;
-    const float hx = sqrtf(Q * q.z / det), hy = sqrtf(Q * q.x / det);
+    const float hx = cull_sqrt<kApprox>(cull_divide<kApprox>(Q * q.z, det));
+    const float hy = cull_sqrt<kApprox>(cull_divide<kApprox>(Q * q.x, det));
     if (!isfinite(hx) || !isfinite(hy)) return s;
     s.mode = 2;
-    s.inv_a = 1.0f / q.x;
+    s.inv_a = cull_divide<kApprox>(1.0f, q.x);
     s.det = det;
     s.qa = q.x * Q;
     s.hy = hy + 0.05f + 1e-3f * hy + 2e-5f * fabsf(mean.y);
-    s.ys = q.y * hx / q.z;
+    s.ys = cull_divide<kApprox>(q.y * hx, q.z);
     s.pad_x = 0.05f + 1e-3f * hx + 2e-5f * fabsf(mean.x);
     return s;
 }
 
 // Columns [x, y) of tile row ty (inside rect) that the record can reach.
-__device__ __noinline__ int2 cull_row_span(CullShape s, int4 rect, int ty) {
+template <bool kApprox>
+__device__ __forceinline__ int2 make_row_span(const CullShape& s, int4 rect, int ty) {
     if (s.mode == 0) return make_int2(rect.x, rect.x);
     if (s.mode == 1) return make_int2(rect.x, rect.z);
     const float y0 = static_cast<float>(ty * kTile) - s.my, y1 = y0 + (kTile - 1);
     if (y0 > s.hy || y1 < -s.hy) return make_int2(rect.x, rect.x);
     const float yr = fminf(fmaxf(-s.ys, y0), y1), yl = fminf(fmaxf(s.ys, y0), y1);
-    const float xr = (-s.B * yr + sqrtf(fmaxf(s.qa - s.det * yr * yr, 0.0f))) * s.inv_a;
-    const float xl = (-s.B * yl - sqrtf(fmaxf(s.qa - s.det * yl * yl, 0.0f))) * s.inv_a;
+    const float xr = (-s.B * yr + cull_sqrt<kApprox>(fmaxf(s.qa - s.det * yr * yr, 0.0f))) * s.inv_a;
+    const float xl = (-s.B * yl - cull_sqrt<kApprox>(fmaxf(s.qa - s.det * yl * yl, 0.0f))) * s.inv_a;
     // tile tx holds pixel centres [16 tx, 16 tx + 15]
     const float c0 = floorf((s.mx + xl - s.pad_x) * (1.0f / kTile));
     const float c1 = floorf((s.mx + xr + s.pad_x) * (1.0f / kTile)) + 1.0f;
@@ -109,11 +129,35 @@ __device__ __noinline__ int2 cull_row_span(CullShape s, int4 rect, int ty) {
     return make_int2(a, max(a, b));
 }
 
-__device__ __forceinline__ int cull_count(float2 mean, float4 q, int4 rect) {
+__device__ __noinline__ CullShape cull_shape(float2 mean, float4 q) { return make_cull_shape<false>(mean, q); }
+
+__device__ __noinline__ int2 cull_row_span(CullShape s, int4 rect, int ty) {
+    return make_row_span<false>(s, rect, ty);
+}
+
+// The records of a Gaussian: their count, and in `kept` its first tile (x in the low
+// 16 bits of .x, y in the high ones), the eight row bytes (.y, .z) and 1 in .w, or 0
+// where the emitter has to find them again.
+__device__ __forceinline__ int cull_count(float2 mean, float4 q, int4 rect, uint4* kept) {
+    const int rows = rect.w - rect.y;
+    *kept = make_uint4(0u, 0u, 0u, 0u);
+    int total = 0;
+    if (rows <= 8 && rect.z - rect.x <= 15 && rect.x < 65536 && rect.y < 65536) {
+        const CullShape s = make_cull_shape<true>(mean, q);
+        uint32_t word[2] = {0u, 0u};
+        for (int r = 0; r < rows; ++r) {
+            const int2 span = make_row_span<true>(s, rect, rect.y + r);
+            const uint32_t byte = static_cast<uint32_t>(span.x - rect.x) | static_cast<uint32_t>(span.y - span.x) << 4;
+            if (r < 4) word[0] |= byte << (8 * r);
+            else word[1] |= byte << (8 * r - 32);
+            total += span.y - span.x;
+        }
+        *kept = make_uint4(static_cast<uint32_t>(rect.x) | static_cast<uint32_t>(rect.y) << 16, word[0], word[1], 1u);
+        return total;
+    }
     const CullShape s = cull_shape(mean, q);
     if (s.mode == 0) return 0;
-    if (s.mode == 1) return (rect.z - rect.x) * (rect.w - rect.y);
-    int total = 0;
+    if (s.mode == 1) return (rect.z - rect.x) * rows;
     for (int ty = rect.y; ty < rect.w; ++ty) {
         const int2 span = cull_row_span(s, rect, ty);
         total += span.y - span.x;
@@ -121,86 +165,123 @@ __device__ __forceinline__ int cull_count(float2 mean, float4 q, int4 rect) {
     return total;
 }
 
-// Records of the culled counts in depth order. Four lanes serve a Gaussian and
-// take its rows four at a time, one row each: a lane finds its row's column
-// interval, the group's exclusive prefix of the interval widths (shuffles
-// within the four lanes) places the row, and the four lanes write the group's
-// records interleaved (consecutive lanes, consecutive slots).
+// 8 lanes per Gaussian here and in emit_records (sort.cu), in resident blocks over the
+// visible ones: with 4 lanes the few records a lane writes at a time left half-written
+// sectors and idle warps (plain 75 -> 68 us and culled 75 -> 67 us at 1.2M Gaussians,
+// culled 39 -> 24 us on 30k large ones, 172 -> 149 us at 3.0M, where 4 lanes take 119).
+constexpr int kEmitLanes = 8;
+
+// Records of the culled counts in depth order. kEmitLanes lanes serve a
+// Gaussian. Where its intervals were kept, each lane writes every kEmitLanes-th record,
+// stepping through the row bytes.
+// Otherwise the first four lanes take its rows four at a time, one row each: a lane
+// finds its row's column interval, the group's exclusive prefix of the interval widths
+// (shuffles) places the row, and all lanes write the group's records interleaved
+// (consecutive lanes, consecutive slots).
 // The loop runs the warp's largest number of row groups so every shuffle sees
 // all 32 lanes.
 __global__ void __launch_bounds__(256) emit_records_culled(const uint32_t* __restrict__ sorted_ids,
                                                            const int* __restrict__ record_start,
+                                                           const uint4* __restrict__ kept_spans,
                                                            const int4* __restrict__ rects,
                                                            const float2* __restrict__ means,
                                                            const float4* __restrict__ conic_opacity, int n,
-                                                           int tile_count_x, uint32_t* __restrict__ tile_keys,
+                                                           const int* __restrict__ visible, int tile_count_x,
+                                                           uint32_t* __restrict__ tile_keys,
                                                            uint32_t* __restrict__ record_ids, int64_t capacity,
                                                            int* overflow) {
     pdl_begin();
-    const int64_t gidx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t p = gidx >> 2;
-    const int sub = static_cast<int>(gidx & 3);
-    bool active = p < n;
-    int begin = 0, count = 0;
-    uint32_t id = 0;
-    if (active) {
-        // the id is loaded with the offsets, ahead of the count checks
-        begin = record_start[p];
-        count = record_start[p + 1] - begin;
-        id = sorted_ids[p];
-        active = count > 0;
-        // past the capacity the overflow flag is set and the records that still
-        // fit are written (below), so every slot below min(total, capacity) -
-        // all the sort and the blend read - holds a record
-        if (active && begin + static_cast<int64_t>(count) > capacity) {
-            if (sub == 0 && overflow) atomicExch(overflow, 1);
-            active = begin < capacity;
+    // the depth order holds the visible Gaussians only
+    const int64_t lanes = static_cast<int64_t>(kEmitLanes) * (visible ? min(*visible, n) : n);
+    const int sub = threadIdx.x % kEmitLanes;
+    for (int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x; first < lanes;
+         first += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t p = (first + threadIdx.x) / kEmitLanes;
+        bool active = first + threadIdx.x < lanes;
+        int begin = 0, count = 0;
+        uint32_t id = 0;
+        if (active) {
+            // the id is loaded with the offsets, ahead of the count checks
+            begin = record_start[p];
+            count = record_start[p + 1] - begin;
+            id = sorted_ids[p];
+            active = count > 0;
+            // past the capacity the overflow flag is set and the records that still
+            // fit are written (below), so every slot below min(total, capacity) -
+            // all the sort and the blend read - holds a record
+            if (active && begin + static_cast<int64_t>(count) > capacity) {
+                if (sub == 0 && overflow) atomicExch(overflow, 1);
+                active = begin < capacity;
+            }
         }
-    }
-    int4 r = make_int4(0, 0, 0, 0);
-    CullShape s{};
-    if (active) {
-        r = rects[id];
-        s = cull_shape(means[id], conic_opacity[id]);
-    }
-    const int groups = active ? (r.w - r.y + 3) / 4 : 0;
-    const int rounds = __reduce_max_sync(0xffffffffu, groups);
-    int k = 0;
-    for (int g = 0; g < rounds; ++g) {
-        const int ty = r.y + 4 * g + sub;
-        int2 span = make_int2(0, 0);
-        if (g < groups && ty < r.w) span = cull_row_span(s, r, ty);
-        const int w = span.y - span.x;
-        // exclusive prefix of the widths over the four lanes of this Gaussian
-        int incl = w;
+        uint4 kept = make_uint4(0u, 0u, 0u, 1u);
+        if (active) kept = kept_spans[id];
+        if (active && kept.w) {
+            const int fit = static_cast<int>(min(static_cast<int64_t>(count), capacity - begin));
+            uint64_t rows = static_cast<uint64_t>(kept.y) | static_cast<uint64_t>(kept.z) << 32;
+            int tile = static_cast<int>(kept.x >> 16) * tile_count_x + static_cast<int>(kept.x & 0xffffu);
+            int before = 0, through = static_cast<int>((rows >> 4) & 15u);  // records before and through this row
+            int left = 8;
+            for (int k = sub; k < fit; k += kEmitLanes) {
+                while (k >= through && --left > 0) {
+                    rows >>= 8;
+                    tile += tile_count_x;
+                    before = through;
+                    through += static_cast<int>((rows >> 4) & 15u);
+                }
+                tile_keys[begin + k] = static_cast<uint32_t>(tile + static_cast<int>(rows & 15u) + k - before);
+                record_ids[begin + k] = id;
+            }
+        }
+        active = active && !kept.w;
+        if (!__any_sync(0xffffffffu, active)) continue;
+        int4 r = make_int4(0, 0, 0, 0);
+        CullShape s{};
+        if (active) {
+            r = rects[id];
+            s = cull_shape(means[id], conic_opacity[id]);
+        }
+        const int groups = active ? (r.w - r.y + 3) / 4 : 0;
+        const int rounds = __reduce_max_sync(0xffffffffu, groups);
+        int k = 0;
+        for (int g = 0; g < rounds; ++g) {
+            const int ty = r.y + 4 * g + sub;
+            int2 span = make_int2(0, 0);
+            if (g < groups && sub < 4 && ty < r.w) span = cull_row_span(s, r, ty);
+            const int w = span.y - span.x;
+            // exclusive prefix of the widths over the four row lanes of this Gaussian
+            int incl = w;
 #pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o, 4);
-            if (sub >= o) incl += y;
+            for (int o = 1; o < 4; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o, kEmitLanes);
+                if (sub >= o) incl += y;
+            }
+            const int group_total = __shfl_sync(0xffffffffu, incl, 3, kEmitLanes);
+            // the group's four rows are one contiguous run of records; a record at
+            // run position q of row i has tile q + base_i. The lanes write the
+            // run interleaved, so consecutive lanes write consecutive slots.
+            const int base = ty * tile_count_x + span.x - (incl - w);
+            const int e0 = __shfl_sync(0xffffffffu, incl, 0, kEmitLanes), e1 = __shfl_sync(0xffffffffu, incl, 1, kEmitLanes);
+            const int e2 = __shfl_sync(0xffffffffu, incl, 2, kEmitLanes);
+            const int b0 = __shfl_sync(0xffffffffu, base, 0, kEmitLanes), b1 = __shfl_sync(0xffffffffu, base, 1, kEmitLanes);
+            const int b2 = __shfl_sync(0xffffffffu, base, 2, kEmitLanes), b3 = __shfl_sync(0xffffffffu, base, 3, kEmitLanes);
+            for (int q = sub; q < group_total && k + q < count && begin + k + q < capacity; q += kEmitLanes) {
+                const int row_base = q < e0 ? b0 : q < e1 ? b1 : q < e2 ? b2 : b3;
+                tile_keys[begin + k + q] = static_cast<uint32_t>(row_base + q);
+                record_ids[begin + k + q] = id;
+            }
+            k += group_total;
         }
-        const int group_total = __shfl_sync(0xffffffffu, incl, 3, 4);
-        // the group's four rows are one contiguous run of records; a record at
-        // run position q of row i has tile q + base_i. The four lanes write the
-        // run interleaved, so consecutive lanes write consecutive slots.
-        const int base = ty * tile_count_x + span.x - (incl - w);
-        const int e0 = __shfl_sync(0xffffffffu, incl, 0, 4), e1 = __shfl_sync(0xffffffffu, incl, 1, 4);
-        const int e2 = __shfl_sync(0xffffffffu, incl, 2, 4);
-        const int b0 = __shfl_sync(0xffffffffu, base, 0, 4), b1 = __shfl_sync(0xffffffffu, base, 1, 4);
-        const int b2 = __shfl_sync(0xffffffffu, base, 2, 4), b3 = __shfl_sync(0xffffffffu, base, 3, 4);
-        for (int q = sub; q < group_total && k + q < count && begin + k + q < capacity; q += 4) {
-            const int row_base = q < e0 ? b0 : q < e1 ? b1 : q < e2 ? b2 : b3;
-            tile_keys[begin + k + q] = static_cast<uint32_t>(row_base + q);
-            record_ids[begin + k + q] = id;
-        }
-        k += group_total;
+        if (active && k != count && sub == 0 && overflow) atomicExch(overflow, 2);
     }
-    if (active && k != count && sub == 0 && overflow) atomicExch(overflow, 2);
 }
 
 // kBf16: precision form (bf16 SH rows; near-singular conics inverted in FP64).
 // TW x TH: tile shape of the rectangle (16 x 16, the reference's, everywhere but
 // the multi-view renderer's tile-shape sweep).
-template <int D, bool kBf16, int TW = kTile, int TH = kTile>
+// kCull: the culled counts too (an instantiation of its own: the span arithmetic costs
+// the plain projection registers, 76 -> 83 us at 1.2M Gaussians).
+template <int D, bool kBf16, bool kCull = false, int TW = kTile, int TH = kTile>
 __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ params,
                                                       gsn_camera cam_arg, const gsn_camera* __restrict__ cam_dev,
                                                       int n, ProjectOutputs out) {
@@ -210,7 +291,7 @@ __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ 
     const gsn_camera cam = cam_dev ? *cam_dev : cam_arg;
     const int64_t N = n;
     out.tile_counts[i] = 0;
-    if (out.cull_counts) out.cull_counts[i] = 0;
+    if (kCull) out.cull_counts[i] = 0;
     out.depth_keys[i] = 0xFFFFFFFFu;
     if (out.radii) out.radii[i] = 0.0f;
 
@@ -303,8 +384,10 @@ __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ 
         conic = make_float4(c * det_inv, -b * det_inv, a * det_inv, opacity);
     }
     out.conic_opacity[i] = conic;
-    if constexpr (TW == kTile && TH == kTile) {
-        if (out.cull_counts) out.cull_counts[i] = cull_count(make_float2(u, v), conic, rect);
+    if constexpr (kCull) {
+        uint4 kept;
+        out.cull_counts[i] = cull_count(make_float2(u, v), conic, rect, &kept);
+        out.cull_spans[i] = kept;
     }
 
     // View direction from the camera centre, C = -R^T t.
@@ -328,15 +411,15 @@ __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ 
     out.colors[i] = make_float3(rgb[0], rgb[1], rgb[2]);
 }
 
-template <bool kBf16>
+template <bool kBf16, bool kCull>
 void launch_project_layout(const float* params, int n, const gsn_camera& cam, const gsn_camera* cam_dev, int d,
                            const ProjectOutputs& out, cudaStream_t stream) {
     dim3 grid(ceil_div(n, 256));
     switch (d) {
-        case 0: launch_step(project_kernel<0, kBf16>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
-        case 1: launch_step(project_kernel<1, kBf16>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
-        case 2: launch_step(project_kernel<2, kBf16>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
-        default: launch_step(project_kernel<3, kBf16>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
+        case 0: launch_step(project_kernel<0, kBf16, kCull>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
+        case 1: launch_step(project_kernel<1, kBf16, kCull>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
+        case 2: launch_step(project_kernel<2, kBf16, kCull>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
+        default: launch_step(project_kernel<3, kBf16, kCull>, grid, 256, 0, stream, params, cam, cam_dev, n, out); break;
     }
 }
 
@@ -347,13 +430,13 @@ static void launch_project_tiles(const float* params, int n, const gsn_camera& c
                           cudaStream_t stream) {
     dim3 grid(ceil_div(n, 256));
     switch (d) {
-        case 0: launch_step(project_kernel<0, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
+        case 0: launch_step(project_kernel<0, false, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
             break;
-        case 1: launch_step(project_kernel<1, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
+        case 1: launch_step(project_kernel<1, false, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
             break;
-        case 2: launch_step(project_kernel<2, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
+        case 2: launch_step(project_kernel<2, false, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
             break;
-        default: launch_step(project_kernel<3, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
+        default: launch_step(project_kernel<3, false, false, TW, TH>, grid, 256, 0, stream, params, cam, nullptr, n, out);
             break;
     }
 }
@@ -369,13 +452,13 @@ int launch_project_tiled(const float* params, int n, const gsn_camera& cam, int 
     return launched(1);
 }
 
-int launch_emit_records_culled(const uint32_t* sorted_ids, const int* record_start, const int4* rects,
-                               const float2* means, const float4* conic_opacity, int n, int tile_count_x,
-                               uint32_t* tile_keys, uint32_t* record_ids, int64_t capacity, int* overflow,
-                               cudaStream_t stream) {
+int launch_emit_records_culled(const uint32_t* sorted_ids, const int* record_start, const uint4* cull_spans,
+                               const int4* rects, const float2* means, const float4* conic_opacity, int n,
+                               const int* visible, int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids,
+                               int64_t capacity, int* overflow, cudaStream_t stream) {
     if (n <= 0) return GSN_OK;
-    launch_step(emit_records_culled, ceil_div(4ll * n, 256), 256, 0, stream, sorted_ids, record_start, rects, means,
-                conic_opacity, n, tile_count_x, tile_keys, record_ids, capacity, overflow);
+    launch_step(emit_records_culled, emit_blocks(kEmitLanes, n), 256, 0, stream, sorted_ids, record_start, cull_spans,
+                rects, means, conic_opacity, n, visible, tile_count_x, tile_keys, record_ids, capacity, overflow);
     return launched(1);
 }
 
@@ -383,8 +466,11 @@ int launch_project(const float* params, int n, const gsn_camera& cam, const gsn_
                    bool bf16_sh, const ProjectOutputs& out, cudaStream_t stream) {
     if (n <= 0) return GSN_OK;
     const int d = sh_degree < 0 ? 0 : (sh_degree > 3 ? 3 : sh_degree);
-    if (bf16_sh) launch_project_layout<true>(params, n, cam, cam_dev, d, out, stream);
-    else launch_project_layout<false>(params, n, cam, cam_dev, d, out, stream);
+    const bool cull = out.cull_counts && out.cull_spans;
+    if (bf16_sh && cull) launch_project_layout<true, true>(params, n, cam, cam_dev, d, out, stream);
+    else if (bf16_sh) launch_project_layout<true, false>(params, n, cam, cam_dev, d, out, stream);
+    else if (cull) launch_project_layout<false, true>(params, n, cam, cam_dev, d, out, stream);
+    else launch_project_layout<false, false>(params, n, cam, cam_dev, d, out, stream);
     return launched(1);
 }
 

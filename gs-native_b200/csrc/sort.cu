@@ -574,38 +574,48 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
 }
 
 // ---------------------------------------------------------------- records
-// Four lanes per Gaussian walk its tile rectangle row-major; the records of one
+constexpr int kEmitLanes = 8;
+
+// kEmitLanes lanes per Gaussian walk its tile rectangle row-major (stepping the column
+// instead of dividing by the width); the records of one
 // Gaussian are contiguous and in the same order as the reference writes them.
 __global__ void __launch_bounds__(256) emit_records(const uint32_t* __restrict__ sorted_ids,
                                                     const int* __restrict__ record_start,
-                                                    const int4* __restrict__ rects, int n, int tile_count_x,
+                                                    const int4* __restrict__ rects, int n,
+                                                    const int* __restrict__ visible, int tile_count_x,
                                                     uint32_t* __restrict__ tile_keys,
                                                     uint32_t* __restrict__ record_ids, int64_t capacity,
                                                     int* overflow) {
     pdl_begin();
-    const int64_t gidx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t p = gidx >> 2;
-    const int sub = static_cast<int>(gidx & 3);
-    if (p >= n) return;
-    const int begin = record_start[p];
-    const int count = record_start[p + 1] - begin;
-    if (count <= 0) return;
-    if (begin + static_cast<int64_t>(count) > capacity) {
-        if (sub == 0 && overflow) atomicExch(overflow, 1);
-        if (begin >= capacity) return;
-    }
-    const uint32_t id = sorted_ids[p];
-    const int4 r = rects[id];
-    const int width = r.z - r.x;
-    // past the capacity the overflow flag is set and the records that still fit
-    // are written, so every slot below min(total, capacity) - all the sort and
-    // the blend read - holds a record
-    const int fit = static_cast<int>(min(static_cast<int64_t>(count), capacity - begin));
-    for (int k = sub; k < fit; k += 4) {
-        int ty = r.y + k / width;
-        int tx = r.x + k % width;
-        tile_keys[begin + k] = static_cast<uint32_t>(ty * tile_count_x + tx);
-        record_ids[begin + k] = id;
+    const int64_t lanes = static_cast<int64_t>(kEmitLanes) * (visible ? min(*visible, n) : n);
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const int sub = threadIdx.x % kEmitLanes;
+    for (int64_t at = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; at < lanes; at += step) {
+        const int64_t p = at / kEmitLanes;
+        const int begin = record_start[p];
+        const int count = record_start[p + 1] - begin;
+        if (count <= 0) continue;
+        if (begin + static_cast<int64_t>(count) > capacity) {
+            if (sub == 0 && overflow) atomicExch(overflow, 1);
+            if (begin >= capacity) continue;
+        }
+        const uint32_t id = sorted_ids[p];
+        const int4 r = rects[id];
+        const int width = r.z - r.x;
+        // past the capacity the overflow flag is set and the records that still fit
+        // are written, so every slot below min(total, capacity) - all the sort and
+        // the blend read - holds a record
+        const int fit = static_cast<int>(min(static_cast<int64_t>(count), capacity - begin));
+        int column = sub, row = r.y * tile_count_x + r.x;  // of record k, and its row's first tile
+        for (int k = sub; k < fit; k += kEmitLanes) {
+            while (column >= width) {
+                column -= width;
+                row += tile_count_x;
+            }
+            tile_keys[begin + k] = static_cast<uint32_t>(row + column);
+            record_ids[begin + k] = id;
+            column += kEmitLanes;
+        }
     }
 }
 
@@ -861,11 +871,16 @@ int launch_exclusive_scan(const int* in, const uint32_t* gather, int* out, int n
     return launched(1);
 }
 
+int emit_blocks(int lanes, int n) {
+    const int64_t blocks = (static_cast<int64_t>(lanes) * n + 255) / 256;
+    return static_cast<int>(blocks < kEmitBlocks ? blocks : kEmitBlocks);
+}
+
 int launch_emit_records(const uint32_t* sorted_ids, const int* record_start, const int4* rects, int n,
-                        int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids, int64_t capacity,
-                        int* overflow, cudaStream_t stream) {
+                        const int* visible, int tile_count_x, uint32_t* tile_keys, uint32_t* record_ids,
+                        int64_t capacity, int* overflow, cudaStream_t stream) {
     if (n <= 0) return GSN_OK;
-    launch_step(emit_records, ceil_div(4ll * n, 256), 256, 0, stream, sorted_ids, record_start, rects, n,
+    launch_step(emit_records, emit_blocks(kEmitLanes, n), 256, 0, stream, sorted_ids, record_start, rects, n, visible,
                 tile_count_x, tile_keys, record_ids, capacity, overflow);
     return launched(1);
 }

@@ -112,7 +112,7 @@ bool MultiViewRenderer::Prepare(View& v, const GaussianBuffers& g, const CameraP
     }
     if (!SortScratch(v.sort_scratch, v.sort_scratch_count, n)) return false;
     gsn::ProjectOutputs po{v.means.get(), v.conic.get(), v.colors.get(), v.depths.get(),
-                           v.rects.get(), v.tile_counts.get(), v.depth_keys[0].get(), nullptr, nullptr, 0};
+                           v.rects.get(), v.tile_counts.get(), v.depth_keys[0].get(), nullptr, nullptr, nullptr, 0};
     if (gsn::launch_project_tiled(g.gaussians_, n, v.cam, config_.tile_w, config_.tile_h, sh_degree, po, stream) !=
         GSN_OK)
         return false;
@@ -145,8 +145,8 @@ bool MultiViewRenderer::Order(View& v, int n, cudaStream_t stream) {
     const int records = static_cast<int>(r);
     bool alt = false;
     if (config_.key_bits == 32) {
-        if (gsn::launch_emit_records(v.by_depth, v.record_start.get(), v.rects.get(), n, v.cam.tile_count_x,
-                                     v.tile_keys[0].get(), v.record_ids[0].get(), v.record_capacity, nullptr,
+        if (gsn::launch_emit_records(v.by_depth, v.record_start.get(), v.rects.get(), n, nullptr,
+                                     v.cam.tile_count_x, v.tile_keys[0].get(), v.record_ids[0].get(), v.record_capacity, nullptr,
                                      stream) != GSN_OK)
             return false;
         if (records > 0 &&

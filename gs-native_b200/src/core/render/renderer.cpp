@@ -106,6 +106,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
         host_records_ = nullptr;
         return false;
     }
+    if (exact_culling_ && !cull_spans_.Reserve(gaussian_capacity_)) return false;
     record_offsets_valid_ = false;
     last_count_ = count;
     const gsn_camera& cam = AsGsnCamera(camera);
@@ -116,7 +117,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     if (count > 0) {
         gsn::ProjectOutputs po{means_.get(), conic_opacities_.get(), colors_.get(), depths_.get(),
                                rects_.get(), tile_counts_.get(), depth_keys_[0].get(), radii_.get(),
-                               exact_culling_ ? cull_counts_.get() : nullptr,
+                               exact_culling_ ? cull_counts_.get() : nullptr, cull_spans_.get(),
                                // the fast forms order depths on 24-bit keys (one radix pass less;
                                // depths equal to 2^-16 relative may swap their blend order)
                                fast_blend_ ? 8 : 0};
@@ -181,13 +182,13 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
         gsn::stage_mark(s, gsn::kStageEmitRecords);
         const int emitted =
             exact_culling_
-                ? gsn::launch_emit_records_culled(by_depth, record_start_.get(), rects_.get(), means_.get(),
-                                                  conic_opacities_.get(), count, camera.tile_count_x_,
-                                                  tile_keys_[0].get(), record_ids_[0].get(), record_capacity_,
-                                                  overflow, s)
-                : gsn::launch_emit_records(by_depth, record_start_.get(), rects_.get(), count, camera.tile_count_x_,
-                                           tile_keys_[0].get(), record_ids_[0].get(), record_capacity_, overflow,
-                                           s);
+                ? gsn::launch_emit_records_culled(by_depth, record_start_.get(), cull_spans_.get(), rects_.get(),
+                                                  means_.get(), conic_opacities_.get(), count, visible,
+                                                  camera.tile_count_x_, tile_keys_[0].get(), record_ids_[0].get(),
+                                                  record_capacity_, overflow, s)
+                : gsn::launch_emit_records(by_depth, record_start_.get(), rects_.get(), count, visible,
+                                           camera.tile_count_x_, tile_keys_[0].get(), record_ids_[0].get(),
+                                           record_capacity_, overflow, s);
         if (emitted != GSN_OK) return false;
         const int max_records = fixed_capacity_ ? static_cast<int>(record_capacity_) : static_cast<int>(records);
         scratch = gsn::radix_sort_scratch(sort_scratch_.get(), static_cast<int>(sort_scratch_count_));

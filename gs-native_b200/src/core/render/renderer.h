@@ -131,6 +131,7 @@ private:
     DeviceArray<int4> rects_;
     DeviceArray<int> tile_counts_;
     DeviceArray<int> cull_counts_;  // exact-culling record counts per Gaussian
+    DeviceArray<uint4> cull_spans_;  // and the kept column intervals behind them
     DeviceArray<uint32_t> depth_keys_[2];
     DeviceArray<uint32_t> depth_ids_[2];
     DeviceArray<int> record_start_;

@@ -124,3 +124,41 @@ def test_training_with_culling_matches_plain():
     c = [float(np.median([r[k] for r in runs[1]])) for k in (0, 1)]
     assert abs(c[0] - p[0]) < 0.35, runs
     assert abs(c[1] - p[1]) <= 0.03 * p[1], runs
+
+
+@pytest.mark.parametrize("spread", [-4.5, -2.5, -0.5])
+@pytest.mark.parametrize("capacity", [0, 700])
+def test_kept_and_recomputed_intervals_emit_the_counted_records(spread, capacity):
+    """Rectangles of a few tiles (intervals kept by the projection), around its limit of
+    8 x 15 tiles and far larger (found again by the emitter), mixed in one frame: every
+    tile's list is the plain list without records that reach none of its pixels, and a
+    capacity below the total leaves only whole records."""
+    t = torch()
+    n = 600
+    params = scenes.random_gaussians(n, 21, mean_sigma=1.0)
+    params[3:6] = np.random.default_rng(4).normal(spread, 0.8, (3, n))
+    cam = scenes.ring_cameras(8, 5.0, 15.0, 403, 301, 350.0, 350.0)[2]
+    p = dev(params)
+    frames = {}
+    for culled in (False, True):
+        r = gsn.Renderer()
+        r.set_exact_culling(culled)
+        if culled and capacity:
+            assert r.set_record_capacity(capacity) == 0
+        img = empty((cam.height, cam.width, 3), t.float32)
+        assert r.render(p.data_ptr(), n, cam, [0, 0, 0], img.data_ptr(), 0) == 0
+        sync()
+        b = r.buffers()
+        offsets = host(b.tile_offsets, np.int64, cam.tiles + 1)
+        frames[culled] = (offsets, host(b.tile_gaussian_ids, np.int32, int(offsets[-1])), img.cpu().numpy(),
+                          int(host(b.overflow, np.int32, 1)[0]))
+    plain, cull = frames[False], frames[True]
+    assert cull[3] == (1 if capacity and plain[0][-1] > 0 and cull[0][-1] == capacity else 0)
+    if not capacity:
+        assert np.array_equal(plain[2], cull[2])
+    for tile in range(cam.tiles):
+        mine = cull[1][cull[0][tile]:cull[0][tile + 1]]
+        full = plain[1][plain[0][tile]:plain[0][tile + 1]]
+        assert np.isin(mine, full).all() and len(np.unique(mine)) == len(mine)
+        rank = {g: k for k, g in enumerate(full)}
+        assert all(rank[a] < rank[b] for a, b in zip(mine, mine[1:]))
