@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
                     const int64_t r0 = base + k * 32;
                     const int off = static_cast<int>(r0 & 31);
                     atomicOr(plane + (r0 >> 5), any << off);
-                    if (off) atomicOr(plane + (r0 >> 5) + 1, any >> (32 - off));
+                    // only where a flag falls there: past the last record the word may not exist
+                    const uint32_t over = off ? any >> (32 - off) : 0u;
+                    if (over) atomicOr(plane + (r0 >> 5) + 1, over);
                 }
             }
         }
