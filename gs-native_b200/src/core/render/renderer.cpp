@@ -215,8 +215,11 @@ bool Renderer::Blend(const gsn_camera& cam, const float* background, float* imag
     cudaStream_t s = stream_;
     checkpoints_used_ = tile_count <= gsn::kCheckpointTiles;
     if (checkpoints_used_ &&
-        !checkpoints_.Reserve(gsn::checkpoint_blocks(record_capacity_, tile_count) * GSN_TILE_SIZE * GSN_TILE_SIZE))
-        return false;
+        !checkpoints_.Reserve(gsn::checkpoint_blocks(record_capacity_, tile_count) * GSN_TILE_SIZE * GSN_TILE_SIZE)) {
+        // without room for them the backward pass walks whole lists
+        checkpoints_used_ = false;
+        cudaGetLastError();
+    }
     gsn::RasterForwardArgs ra;
     ra.tile_ids = sorted_ids_;
     ra.tile_offsets = tile_offsets_.get();
