@@ -94,8 +94,11 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     const int lane = threadIdx.x;
     const int tile = blockIdx.x;
     const int64_t begin = a.tile_offsets[tile];
-    // records [0, bound) hold every record a pixel of the tile took
-    const int bound = a.tile_bounds[tile];
+    // records [0, bound) hold every record a pixel of the tile took; within the tile's
+    // list also where the camera has tiles that the last frame had not, whose bounds and
+    // offsets are of different frames
+    const int bound = static_cast<int>(
+        min(static_cast<int64_t>(a.tile_bounds[tile]), a.tile_offsets[tile + 1] - begin));
     // this warp's segment of it: kSegment records, the last warp's to the end
     const int from = static_cast<int>(blockIdx.y) * kSegment;
     if (from >= bound) return;

@@ -213,11 +213,11 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 // The per-tile blend of the ordered records.
 bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
-    checkpoints_used_ = tile_count <= gsn::kCheckpointTiles;
-    if (checkpoints_used_ &&
+    checkpoint_tiles_ = tile_count <= gsn::kCheckpointTiles ? tile_count : 0;
+    if (checkpoint_tiles_ &&
         !checkpoints_.Reserve(gsn::checkpoint_blocks(record_capacity_, tile_count) * GSN_TILE_SIZE * GSN_TILE_SIZE)) {
         // without room for them the backward pass walks whole lists
-        checkpoints_used_ = false;
+        checkpoint_tiles_ = 0;
         cudaGetLastError();
     }
     gsn::RasterForwardArgs ra;
@@ -235,7 +235,7 @@ bool Renderer::Blend(const gsn_camera& cam, const float* background, float* imag
     ra.record_words = record_words_;
     ra.fast = fast_blend_;
     ra.tile_bounds = tile_bounds_.get();
-    ra.checkpoints = checkpoints_used_ ? checkpoints_.get() : nullptr;
+    ra.checkpoints = checkpoint_tiles_ ? checkpoints_.get() : nullptr;
     ra.pair_count = pair_counter_;
     if (record_warps_.get() &&
         cudaMemsetAsync(record_warps_.get(), 0, 2 * static_cast<size_t>(record_words_) * sizeof(uint32_t), s) !=

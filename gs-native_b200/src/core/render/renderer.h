@@ -92,9 +92,12 @@ public:
     int64_t GetRecordWords() const { return record_words_; }
     // Per tile of the last frame, the largest contributor count of its pixels.
     const int* GetTileBounds() const { return tile_bounds_.get(); }
-    // Per-pixel blend states inside long lists, kept for frames of few tiles (null
-    // otherwise): the backward pass starts its segments from them.
-    const float4* GetCheckpoints() const { return checkpoints_used_ ? checkpoints_.get() : nullptr; }
+    // Per-pixel blend states inside long lists, kept for frames of few tiles: the
+    // backward pass starts its segments from them. Null where the last frame kept none
+    // or had another number of tiles.
+    const float4* GetCheckpoints(int64_t tiles) const {
+        return checkpoint_tiles_ == tiles ? checkpoints_.get() : nullptr;
+    }
     const int* GetRecordCountDevice() const { return counters_.get(); }
     const int* GetOverflowFlag() const { return counters_.get() + 1; }
     int64_t GetRecordCapacity() const { return record_capacity_; }
@@ -145,7 +148,7 @@ private:
     DeviceArray<uint32_t> record_warps_;
     DeviceArray<int> tile_bounds_;
     DeviceArray<float4> checkpoints_;
-    bool checkpoints_used_ = false;
+    int checkpoint_tiles_ = 0;  // of the last frame, 0 where it kept none
     int64_t record_words_ = 0;
     size_t pixel_capacity_ = 0;
     DeviceArray<unsigned char> sort_scratch_;

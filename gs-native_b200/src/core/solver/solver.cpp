@@ -134,7 +134,7 @@ bool Solver::ComputeScreenGradients(const CameraParams& camera, const Renderer& 
     a.record_warps = renderer.GetRecordWarps();
     a.record_words = renderer.GetRecordWords();
     a.tile_bounds = renderer.GetTileBounds();
-    a.checkpoints = renderer.GetCheckpoints();
+    a.checkpoints = renderer.GetCheckpoints(tiles);
     a.fast = renderer.GetFastBlend();
     a.cam = AsGsnCamera(camera);
     a.grad_out = screen_.get();
