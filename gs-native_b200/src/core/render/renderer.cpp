@@ -13,6 +13,8 @@ namespace gs_native {
 
 namespace {
 
+constexpr size_t kBlockPixels = static_cast<size_t>(GSN_TILE_SIZE) * GSN_TILE_SIZE;  // of a checkpoint block
+
 int TileBits(int tile_count) {
     int bits = 0;
     for (unsigned int t = static_cast<unsigned int>(tile_count - 1); t; t >>= 1) ++bits;
@@ -67,6 +69,53 @@ bool Renderer::ReserveRecords(int64_t records) {
     return true;
 }
 
+bool Renderer::ReserveSort(int64_t count) {
+    if (static_cast<size_t>(count) <= sort_scratch_count_ && sort_scratch_.get()) return true;
+    const size_t want = std::max<size_t>(count, sort_scratch_count_ + sort_scratch_count_ / 2);
+    if (!sort_scratch_.Reserve(gsn::radix_sort_scratch_bytes(static_cast<int>(std::min<size_t>(want, INT_MAX)))))
+        return false;
+    sort_scratch_count_ = want;
+    return true;
+}
+
+bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
+    if (!ReserveGaussians(count)) return false;
+    if (static_cast<size_t>(tile_count) > tile_capacity_) {
+        if (!tile_offsets_.Reserve(static_cast<size_t>(tile_count) + 1) ||
+            !tile_bounds_.Reserve(static_cast<size_t>(tile_count)))
+            return false;
+        tile_capacity_ = static_cast<size_t>(tile_count);
+    }
+    if (pixels > pixel_capacity_) {
+        if (!contributors_.Reserve(pixels)) return false;
+        pixel_capacity_ = pixels;
+    }
+    if (!fixed_capacity_ && !ReserveRecords(std::max<int64_t>(record_capacity_, 1))) return false;
+    if (!ReserveSort(std::max<int64_t>(count, record_capacity_))) return false;
+    if (static_cast<size_t>(count) > scan_scratch_count_ || !scan_scratch_.get()) {
+        if (!scan_scratch_.Reserve(gsn::scan_scratch_bytes(std::max(count, 1)))) return false;
+        scan_scratch_count_ = static_cast<size_t>(std::max(count, 1));
+    }
+    return !exact_culling_ || cull_spans_.Reserve(gaussian_capacity_);
+}
+
+// Without checkpoints the backward pass walks whole lists, so a frame goes on where
+// there is no memory for them, and does not ask again for as much: every later frame
+// would pay for the failing call. Nothing is allocated while the stream is captured,
+// where cudaMalloc would end the capture.
+void Renderer::ReserveCheckpoints(int tile_count) {
+    if (tile_count > gsn::kCheckpointTiles) return;
+    const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tile_count);
+    if (blocks * kBlockPixels <= checkpoints_.capacity() || (checkpoint_refused_ && blocks >= checkpoint_refused_))
+        return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream_, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+    if (!checkpoints_.Reserve(blocks * kBlockPixels)) {
+        checkpoint_refused_ = blocks;
+        cudaGetLastError();
+    }
+}
+
 bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& camera, const float* background,
                       float* image, int sh_degree) {
     const int count = gaussians.gaussian_count_;
@@ -78,35 +127,13 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     if (tile_count_long >= INT_MAX) return false;
     const int tile_count = static_cast<int>(tile_count_long);
     sh_degree = std::clamp(sh_degree, 0, 3);
-    if (!ReserveGaussians(count)) return false;
-    if (static_cast<size_t>(tile_count) > tile_capacity_) {
-        if (!tile_offsets_.Reserve(static_cast<size_t>(tile_count) + 1) ||
-            !tile_bounds_.Reserve(static_cast<size_t>(tile_count)))
-            return false;
-        tile_capacity_ = static_cast<size_t>(tile_count);
-    }
     const size_t pixels = static_cast<size_t>(camera.width_) * camera.height_;
-    if (pixels > pixel_capacity_) {
-        if (!contributors_.Reserve(pixels)) return false;
-        pixel_capacity_ = pixels;
-    }
-    if (!fixed_capacity_ && !ReserveRecords(std::max<int64_t>(record_capacity_, 1))) return false;
+    if (!ReserveFrame(count, tile_count, pixels)) return false;
     const int sort_max = static_cast<int>(std::max<int64_t>(count, record_capacity_));
-    if (static_cast<size_t>(sort_max) > sort_scratch_count_ || !sort_scratch_.get()) {
-        size_t want = std::max<size_t>(sort_max, sort_scratch_count_ + sort_scratch_count_ / 2);
-        if (!sort_scratch_.Reserve(gsn::radix_sort_scratch_bytes(static_cast<int>(std::min<size_t>(want, INT_MAX)))))
-            return false;
-        sort_scratch_count_ = want;
-    }
-    if (static_cast<size_t>(count) > scan_scratch_count_ || !scan_scratch_.get()) {
-        if (!scan_scratch_.Reserve(gsn::scan_scratch_bytes(std::max(count, 1)))) return false;
-        scan_scratch_count_ = static_cast<size_t>(std::max(count, 1));
-    }
     if (!host_records_ && cudaMallocHost(&host_records_, sizeof(int)) != cudaSuccess) {
         host_records_ = nullptr;
         return false;
     }
-    if (exact_culling_ && !cull_spans_.Reserve(gaussian_capacity_)) return false;
     record_offsets_valid_ = false;
     last_count_ = count;
     const gsn_camera& cam = AsGsnCamera(camera);
@@ -143,6 +170,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
             cudaSuccess)
             return false;
     }
+    ReserveCheckpoints(tile_count);
     return Blend(cam, background, image, tile_count);
 }
 
@@ -171,12 +199,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
                 return false;
             records = *host_records_;
             if (records < 0) return false;
-            if (!ReserveRecords(records)) return false;
-            if (static_cast<size_t>(records) > sort_scratch_count_) {
-                size_t want = std::max<size_t>(records, sort_scratch_count_ + sort_scratch_count_ / 2);
-                if (!sort_scratch_.Reserve(gsn::radix_sort_scratch_bytes(static_cast<int>(want)))) return false;
-                sort_scratch_count_ = want;
-            }
+            if (!ReserveRecords(records) || !ReserveSort(records)) return false;
             last_records_ = records;
         }
         gsn::stage_mark(s, gsn::kStageEmitRecords);
@@ -213,13 +236,9 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 // The per-tile blend of the ordered records.
 bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
-    checkpoint_tiles_ = tile_count <= gsn::kCheckpointTiles ? tile_count : 0;
-    if (checkpoint_tiles_ &&
-        !checkpoints_.Reserve(gsn::checkpoint_blocks(record_capacity_, tile_count) * GSN_TILE_SIZE * GSN_TILE_SIZE)) {
-        // without room for them the backward pass walks whole lists
-        checkpoint_tiles_ = 0;
-        cudaGetLastError();
-    }
+    const bool checkpoints = tile_count <= gsn::kCheckpointTiles &&
+                             gsn::checkpoint_blocks(record_capacity_, tile_count) * kBlockPixels <= checkpoints_.capacity();
+    checkpoint_tiles_ = checkpoints ? tile_count : 0;
     gsn::RasterForwardArgs ra;
     ra.tile_ids = sorted_ids_;
     ra.tile_offsets = tile_offsets_.get();

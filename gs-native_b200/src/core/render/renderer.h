@@ -108,6 +108,11 @@ public:
 private:
     bool ReserveGaussians(int count);
     bool ReserveRecords(int64_t records);
+    bool ReserveSort(int64_t count);
+    // Every buffer of a frame that does not depend on its record count.
+    bool ReserveFrame(int count, int tile_count, size_t pixels);
+    // Room for a frame's checkpoints, where there is memory for them.
+    void ReserveCheckpoints(int tile_count);
 
     cudaStream_t stream_ = nullptr;
     size_t gaussian_capacity_ = 0;
@@ -148,7 +153,8 @@ private:
     DeviceArray<uint32_t> record_warps_;
     DeviceArray<int> tile_bounds_;
     DeviceArray<float4> checkpoints_;
-    int checkpoint_tiles_ = 0;  // of the last frame, 0 where it kept none
+    int checkpoint_tiles_ = 0;        // of the last frame, 0 where it kept none
+    size_t checkpoint_refused_ = 0;  // blocks there was no memory for (0: none refused)
     int64_t record_words_ = 0;
     size_t pixel_capacity_ = 0;
     DeviceArray<unsigned char> sort_scratch_;

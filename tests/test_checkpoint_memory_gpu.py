@@ -1,0 +1,101 @@
+"""The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
+capture go on where there is none, without asking for it again.
+Allocations are counted and refused on the host, through the library's allocation hook."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import gsn
+import scenes
+from helpers import dev, empty, host, sync, torch
+from test_backward_segments_gpu import faint_scene
+
+pytestmark = pytest.mark.gpu
+
+HOOK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t)
+CUDA_ERROR_MEMORY_ALLOCATION = 2
+W, H, COUNT, CAPACITY = 64, 48, 1500, 1 << 20
+# (CAPACITY / 128 + tiles) blocks of 256 float4: 32 MB; every other buffer here is below 5 MB
+LARGE = 16 << 20
+
+
+class Allocations:
+    """Sizes of the library's device allocations while the context is open; `refuse` says
+    which of them fail."""
+
+    def __init__(self, refuse=lambda size: False):
+        self.refuse, self.sizes = refuse, []
+        self.alloc = ctypes.CDLL("libcuda.so.1").cuMemAlloc_v2
+        self.alloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+        self.set = getattr(gsn.lib(), "_ZN9gs_native18SetDeviceAllocHookEPF9cudaErrorPPvmE")
+        self.set.argtypes = [ctypes.c_void_p]
+        self.set.restype = None
+        self.hook = HOOK(self.call)
+
+    def call(self, pointer, size):
+        self.sizes.append(size)
+        if self.refuse(size):
+            return CUDA_ERROR_MEMORY_ALLOCATION
+        return 0 if self.alloc(pointer, size) == 0 else CUDA_ERROR_MEMORY_ALLOCATION
+
+    def __enter__(self):
+        self.set(ctypes.cast(self.hook, ctypes.c_void_p))
+        return self
+
+    def __exit__(self, *_):
+        self.set(None)
+
+    def large(self):
+        return sum(s > LARGE for s in self.sizes)
+
+
+def scene():
+    params = faint_scene(COUNT, 3)
+    cam = scenes.make_camera(W, H, fx=60.0, fy=60.0)
+    target = np.random.default_rng(4).integers(0, 256, (H, W, 3), dtype=np.uint8)
+    return dev(params), cam, dev(target)
+
+
+def gradients(renderer, solver, p, cam, target, image):
+    assert renderer.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
+    solver.image_gradients(cam, image.data_ptr(), target.data_ptr())
+    ptr = solver.screen_gradients(cam, renderer, image.data_ptr(), p.data_ptr(), COUNT)
+    sync()
+    return host(ptr, np.float32, 12 * COUNT).reshape(COUNT, 12)
+
+
+def close(a, b):
+    # the same fp32 terms, summed in float atomics over segments or whole lists
+    scale = np.abs(b).max(0)
+    return np.all(np.abs(a - b) <= 1e-4 * np.abs(b) + 1e-5 * scale)
+
+
+def steps():
+    """Three eager frames with gradients, a capture and three replays."""
+    t = torch()
+    p, cam, target = scene()
+    image = empty((H, W, 3), t.float32)
+    r, s, g = gsn.Renderer(), gsn.Solver(), gsn.Graph()
+    assert r.set_record_capacity(CAPACITY) == 0
+    screens = [gradients(r, s, p, cam, target, image) for _ in range(3)]
+    g.capture(r, s, p.data_ptr(), COUNT, [cam], target.data_ptr(), W * H * 3, [0, 0, 0], image.data_ptr(), 0, CAPACITY)
+    g.run([0, 0, 0], [1e-4] * 3)
+    status = g.check()
+    out = screens, p.cpu().numpy(), status
+    g.close()
+    return out
+
+
+def test_a_step_and_a_capture_go_on_without_checkpoints():
+    screens, params, status = steps()
+    with Allocations(lambda size: size > LARGE) as none:
+        without, params_without, status_without = steps()
+    assert none.large() == 1  # asked for once, not per frame and not inside the capture
+    assert status == status_without == 0
+    for a, b in zip(without, screens):
+        assert close(a, b)
+    start = scene()[0].cpu().numpy()
+    moved = np.abs(params - start)
+    assert moved.max() > 0
+    assert np.mean(np.abs(params_without - params) <= 1e-6 + 1e-3 * moved) > 0.999
