@@ -102,10 +102,13 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
 // Without checkpoints the backward pass walks whole lists, so a frame goes on where
 // there is no memory for them, and does not ask again for as much: every later frame
 // would pay for the failing call. Nothing is allocated while the stream is captured,
-// where cudaMalloc would end the capture.
+// where cudaMalloc would end the capture. Sized for the tiles reserved so far, the
+// buffer moves only when tile_offsets_ or the record buffers do, so that a graph
+// captured over them outlives eager frames of other sizes.
 void Renderer::ReserveCheckpoints(int tile_count) {
     if (tile_count > gsn::kCheckpointTiles) return;
-    const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tile_count);
+    const int tiles = static_cast<int>(std::min<size_t>(tile_capacity_, gsn::kCheckpointTiles));
+    const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tiles);
     if (blocks * kBlockPixels <= checkpoints_.capacity() || (checkpoint_refused_ && blocks >= checkpoint_refused_))
         return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;

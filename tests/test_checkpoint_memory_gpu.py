@@ -1,5 +1,6 @@
 """The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
-capture go on where there is none, without asking for it again.
+capture go on where there is none, without asking for it again, and the buffer stays
+where it is for frames that need no more room.
 Allocations are counted and refused on the host, through the library's allocation hook."""
 import ctypes
 
@@ -99,3 +100,21 @@ def test_a_step_and_a_capture_go_on_without_checkpoints():
     moved = np.abs(params - start)
     assert moved.max() > 0
     assert np.mean(np.abs(params_without - params) <= 1e-6 + 1e-3 * moved) > 0.999
+
+
+def test_checkpoints_stay_in_place_for_frames_of_fewer_tiles_than_reserved():
+    t = torch()
+    p, cam, target = scene()
+    r, s = gsn.Renderer(), gsn.Solver()
+    assert r.set_record_capacity(CAPACITY) == 0
+    image = empty((1024, 1040, 3), t.float32)
+    wide = scenes.make_camera(1040, 1024, fx=60.0, fy=60.0)  # 65 x 64 tiles: keeps none
+    middle = scenes.make_camera(800, 700, fx=60.0, fy=60.0)
+    big_target = empty((1024, 1040, 3), t.uint8)
+    gradients(r, s, p, wide, big_target, image)
+    for _ in range(2):
+        gradients(r, s, p, cam, target, image)
+    with Allocations() as seen:
+        gradients(r, s, p, middle, big_target, image)
+        gradients(r, s, p, cam, target, image)
+    assert seen.sizes == []
