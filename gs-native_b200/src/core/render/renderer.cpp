@@ -119,6 +119,19 @@ void Renderer::ReserveCheckpoints(int tile_count) {
     }
 }
 
+// The frame's own buffers come before the checkpoints. Not with a fixed capacity: a
+// captured graph may hold their address.
+template <typename Reserve>
+bool Renderer::ReserveAtAnyRate(Reserve reserve) {
+    if (reserve()) return true;
+    if (fixed_capacity_ || !checkpoints_.get()) return false;
+    cudaGetLastError();
+    checkpoint_refused_ = 1;
+    checkpoint_tiles_ = 0;
+    checkpoints_.Reset();
+    return reserve();
+}
+
 bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& camera, const float* background,
                       float* image, int sh_degree) {
     const int count = gaussians.gaussian_count_;
@@ -131,7 +144,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     const int tile_count = static_cast<int>(tile_count_long);
     sh_degree = std::clamp(sh_degree, 0, 3);
     const size_t pixels = static_cast<size_t>(camera.width_) * camera.height_;
-    if (!ReserveFrame(count, tile_count, pixels)) return false;
+    if (!ReserveAtAnyRate([&] { return ReserveFrame(count, tile_count, pixels); })) return false;
     const int sort_max = static_cast<int>(std::max<int64_t>(count, record_capacity_));
     if (!host_records_ && cudaMallocHost(&host_records_, sizeof(int)) != cudaSuccess) {
         host_records_ = nullptr;
@@ -202,7 +215,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
                 return false;
             records = *host_records_;
             if (records < 0) return false;
-            if (!ReserveRecords(records) || !ReserveSort(records)) return false;
+            if (!ReserveAtAnyRate([&] { return ReserveRecords(records) && ReserveSort(records); })) return false;
             last_records_ = records;
         }
         gsn::stage_mark(s, gsn::kStageEmitRecords);

@@ -113,6 +113,9 @@ private:
     bool ReserveFrame(int count, int tile_count, size_t pixels);
     // Room for a frame's checkpoints, where there is memory for them.
     void ReserveCheckpoints(int tile_count);
+    // reserve() again without the checkpoints, where it fails with them.
+    template <typename Reserve>
+    bool ReserveAtAnyRate(Reserve reserve);
 
     cudaStream_t stream_ = nullptr;
     size_t gaussian_capacity_ = 0;

@@ -1,6 +1,6 @@
 """The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
-capture go on where there is none, without asking for it again, and the buffer stays
-where it is for frames that need no more room.
+capture go on where there is none, without asking for it again; the buffer stays where
+it is for frames that need no more room; and a frame's own buffers come before it.
 Allocations are counted and refused on the host, through the library's allocation hook."""
 import ctypes
 
@@ -118,3 +118,29 @@ def test_checkpoints_stay_in_place_for_frames_of_fewer_tiles_than_reserved():
         gradients(r, s, p, middle, big_target, image)
         gradients(r, s, p, cam, target, image)
     assert seen.sizes == []
+
+
+def test_the_frames_own_buffers_come_before_checkpoints():
+    t = torch()
+    p, cam, target = scene()
+    image = empty((H, W, 3), t.float32)
+    r, s = gsn.Renderer(), gsn.Solver()
+    for _ in range(2):
+        gradients(r, s, p, cam, target, image)  # grow mode, checkpoints held
+    n = 40000
+    more = dev(faint_scene(n, 8))
+    fresh = gsn.Renderer()
+    expected, got = empty((H, W, 3), t.float32), empty((H, W, 3), t.float32)
+    assert fresh.render(more.data_ptr(), n, cam, [0, 0, 0], expected.data_ptr(), 0) == 0
+    refusals = []
+
+    def once(size):  # as if the memory that checkpoints hold were the last
+        if size > 1 << 17 and not refusals:
+            refusals.append(size)
+            return True
+        return False
+
+    with Allocations(once):
+        assert r.render(more.data_ptr(), n, cam, [0, 0, 0], got.data_ptr(), 0) == 0
+    sync()
+    assert refusals and torch().equal(expected, got)
