@@ -63,6 +63,7 @@ bool TrainingGraph::Capture(Renderer& renderer, Solver& solver, GaussianBuffers&
     renderer.SetStream(stream);
     solver.SetStream(stream);
     if (!renderer.SetRecordCapacity(record_capacity)) return false;
+    renderer.KeepCheckpoints(static_cast<int64_t>(c0.tile_count_x_) * c0.tile_count_y_);
     // eager pass without the update: every buffer of the step is reserved
     // before the capture, which must not allocate or synchronise
     if (!renderer.Render(gaussians, c0, background, device_image, sh_degree) ||

@@ -105,9 +105,9 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
 // where cudaMalloc would end the capture. Sized for the tiles reserved so far, the
 // buffer moves only when tile_offsets_ or the record buffers do, so that a graph
 // captured over them outlives eager frames of other sizes.
-void Renderer::ReserveCheckpoints(int tile_count) {
-    if (tile_count > gsn::kCheckpointTiles) return;
-    const int tiles = static_cast<int>(std::min<size_t>(tile_capacity_, gsn::kCheckpointTiles));
+void Renderer::ReserveCheckpoints(int64_t tile_count) const {
+    if (!keep_checkpoints_.load() || tile_count > gsn::kCheckpointTiles) return;
+    const int tiles = std::min(std::max(static_cast<int>(tile_count), GetTileCapacity()), gsn::kCheckpointTiles);
     const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tiles);
     if (blocks * kBlockPixels <= checkpoints_.capacity() || (checkpoint_refused_ && blocks >= checkpoint_refused_))
         return;
@@ -117,6 +117,11 @@ void Renderer::ReserveCheckpoints(int tile_count) {
         checkpoint_refused_ = blocks;
         cudaGetLastError();
     }
+}
+
+// Reserves at once, so that one step is enough of a warm-up before a capture.
+void Renderer::KeepCheckpoints(int64_t tiles) const {
+    if (!keep_checkpoints_.exchange(true)) ReserveCheckpoints(tiles);
 }
 
 // The frame's own buffers come before the checkpoints. Not with a fixed capacity: a
@@ -252,7 +257,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 // The per-tile blend of the ordered records.
 bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
-    const bool checkpoints = tile_count <= gsn::kCheckpointTiles &&
+    const bool checkpoints = keep_checkpoints_.load() && tile_count <= gsn::kCheckpointTiles &&
                              gsn::checkpoint_blocks(record_capacity_, tile_count) * kBlockPixels <= checkpoints_.capacity();
     checkpoint_tiles_ = checkpoints ? tile_count : 0;
     gsn::RasterForwardArgs ra;

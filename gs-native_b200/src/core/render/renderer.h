@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
@@ -92,6 +93,10 @@ public:
     int64_t GetRecordWords() const { return record_words_; }
     // Per tile of the last frame, the largest contributor count of its pixels.
     const int* GetTileBounds() const { return tile_bounds_.get(); }
+    // A backward pass reads this renderer's frames: those after the call keep checkpoints
+    // (the solver calls it; before it a renderer, which may only ever render, holds none).
+    // `tiles`: of the last frame.
+    void KeepCheckpoints(int64_t tiles) const;
     // Per-pixel blend states inside long lists, kept for frames of few tiles: the
     // backward pass starts its segments from them. Null where the last frame kept none
     // or had another number of tiles.
@@ -112,7 +117,7 @@ private:
     // Every buffer of a frame that does not depend on its record count.
     bool ReserveFrame(int count, int tile_count, size_t pixels);
     // Room for a frame's checkpoints, where there is memory for them.
-    void ReserveCheckpoints(int tile_count);
+    void ReserveCheckpoints(int64_t tile_count) const;
     // reserve() again without the checkpoints, where it fails with them.
     template <typename Reserve>
     bool ReserveAtAnyRate(Reserve reserve);
@@ -155,9 +160,10 @@ private:
     DeviceArray<int> contributors_;
     DeviceArray<uint32_t> record_warps_;
     DeviceArray<int> tile_bounds_;
-    DeviceArray<float4> checkpoints_;
-    int checkpoint_tiles_ = 0;        // of the last frame, 0 where it kept none
-    size_t checkpoint_refused_ = 0;  // blocks there was no memory for (0: none refused)
+    mutable std::atomic<bool> keep_checkpoints_{false};
+    mutable DeviceArray<float4> checkpoints_;
+    int checkpoint_tiles_ = 0;  // of the last frame, 0 where it kept none
+    mutable size_t checkpoint_refused_ = 0;  // blocks there was no memory for (0: none refused)
     int64_t record_words_ = 0;
     size_t pixel_capacity_ = 0;
     DeviceArray<unsigned char> sort_scratch_;

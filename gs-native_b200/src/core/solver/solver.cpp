@@ -119,6 +119,7 @@ bool Solver::ComputeScreenGradients(const CameraParams& camera, const Renderer& 
     if (count != gaussian_count_) {
         if (iteration_ != 0 || !RemapGaussians(nullptr, count)) return false;
     }
+    renderer.KeepCheckpoints(tiles);
     gsn::stage_mark(stream_, gsn::kStageRasterBackward);
     if (cudaMemsetAsync(screen_.get(), 0, static_cast<size_t>(count) * 12 * sizeof(float), stream_) != cudaSuccess)
         return false;

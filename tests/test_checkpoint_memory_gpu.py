@@ -1,6 +1,7 @@
 """The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
 capture go on where there is none, without asking for it again; the buffer stays where
-it is for frames that need no more room; and a frame's own buffers come before it.
+it is for frames that need no more room; a frame's own buffers come before it; and a
+renderer whose frames no backward pass reads has none.
 Allocations are counted and refused on the host, through the library's allocation hook."""
 import ctypes
 
@@ -144,3 +145,21 @@ def test_the_frames_own_buffers_come_before_checkpoints():
         assert r.render(more.data_ptr(), n, cam, [0, 0, 0], got.data_ptr(), 0) == 0
     sync()
     assert refusals and torch().equal(expected, got)
+
+
+def test_a_renderer_that_only_renders_keeps_no_checkpoints():
+    t = torch()
+    p, cam, target = scene()
+    image = empty((H, W, 3), t.float32)
+    r, s = gsn.Renderer(), gsn.Solver()
+    with Allocations() as seen:
+        assert r.set_record_capacity(CAPACITY) == 0
+        for _ in range(3):
+            assert r.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
+        sync()
+        assert seen.large() == 0
+        whole = gradients(r, s, p, cam, target, image)
+        assert seen.large() == 1  # by the first backward pass, for the next frame
+        segments = gradients(r, s, p, cam, target, image)
+        assert seen.large() == 1
+    assert close(whole, segments)
