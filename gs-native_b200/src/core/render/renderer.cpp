@@ -46,7 +46,7 @@ bool Renderer::ReserveGaussians(int count) {
     size_t grow = std::max(n, gaussian_capacity_ + gaussian_capacity_ / 4);
     bool ok = means_.Reserve(grow) && conic_opacities_.Reserve(grow) && colors_.Reserve(grow) &&
               depths_.Reserve(grow) && radii_.Reserve(grow) && rects_.Reserve(grow) &&
-              tile_counts_.Reserve(grow) && cull_counts_.Reserve(grow) && depth_keys_[0].Reserve(grow) &&
+              tile_counts_.Reserve(grow) && depth_keys_[0].Reserve(grow) &&
               depth_keys_[1].Reserve(grow) &&
               depth_ids_[0].Reserve(grow) && depth_ids_[1].Reserve(grow) && record_start_.Reserve(grow + 1) &&
               counters_.Reserve(3);
@@ -81,9 +81,8 @@ bool Renderer::ReserveSort(int64_t count) {
 bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
     if (!ReserveGaussians(count)) return false;
     if (static_cast<size_t>(tile_count) > tile_capacity_) {
-        if (!tile_offsets_.Reserve(static_cast<size_t>(tile_count) + 1) ||
-            !tile_bounds_.Reserve(static_cast<size_t>(tile_count)))
-            return false;
+        const size_t tiles = static_cast<size_t>(tile_count);
+        if (!tile_offsets_.Reserve(tiles + 1 + (tiles + 1) / 2)) return false;
         tile_capacity_ = static_cast<size_t>(tile_count);
     }
     if (pixels > pixel_capacity_) {
@@ -96,7 +95,7 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
         if (!scan_scratch_.Reserve(gsn::scan_scratch_bytes(std::max(count, 1)))) return false;
         scan_scratch_count_ = static_cast<size_t>(std::max(count, 1));
     }
-    return !exact_culling_ || cull_spans_.Reserve(gaussian_capacity_);
+    return !exact_culling_ || cull_spans_.Reserve(gaussian_capacity_ + (gaussian_capacity_ + 3) / 4);
 }
 
 // Without checkpoints the backward pass walks whole lists, so a frame goes on where
@@ -165,7 +164,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     if (count > 0) {
         gsn::ProjectOutputs po{means_.get(), conic_opacities_.get(), colors_.get(), depths_.get(),
                                rects_.get(), tile_counts_.get(), depth_keys_[0].get(), radii_.get(),
-                               exact_culling_ ? cull_counts_.get() : nullptr, cull_spans_.get(),
+                               exact_culling_ ? CullCounts() : nullptr, cull_spans_.get(),
                                // the fast forms order depths on 24-bit keys (one radix pass less;
                                // depths equal to 2^-16 relative may swap their blend order)
                                fast_blend_ ? 8 : 0};
@@ -207,7 +206,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
     bool in_alt = false;
     {
         gsn::stage_mark(s, gsn::kStageRecordScan);
-        if (gsn::launch_exclusive_scan(exact_culling_ ? cull_counts_.get() : tile_counts_.get(), by_depth,
+        if (gsn::launch_exclusive_scan(exact_culling_ ? CullCounts() : tile_counts_.get(), by_depth,
                                        record_start_.get(), count, scan_scratch_.get(), s, visible) != GSN_OK)
             return false;
         if (cudaMemcpyAsync(record_count, record_start_.get() + count, sizeof(int), cudaMemcpyDeviceToDevice,
@@ -274,7 +273,7 @@ bool Renderer::Blend(const gsn_camera& cam, const float* background, float* imag
     ra.record_warps = record_warps_.get();
     ra.record_words = record_words_;
     ra.fast = fast_blend_;
-    ra.tile_bounds = tile_bounds_.get();
+    ra.tile_bounds = TileBounds();
     ra.checkpoints = checkpoint_tiles_ ? checkpoints_.get() : nullptr;
     ra.pair_count = pair_counter_;
     if (record_warps_.get() &&

@@ -92,7 +92,7 @@ public:
     const uint32_t* GetRecordWarps() const { return record_warps_.get(); }
     int64_t GetRecordWords() const { return record_words_; }
     // Per tile of the last frame, the largest contributor count of its pixels.
-    const int* GetTileBounds() const { return tile_bounds_.get(); }
+    const int* GetTileBounds() const { return TileBounds(); }
     // A backward pass reads this renderer's frames: those after the call keep checkpoints
     // (the solver calls it; before it a renderer, which may only ever render, holds none).
     // `tiles`: of the last frame.
@@ -146,20 +146,23 @@ private:
     DeviceArray<float> radii_;
     DeviceArray<int4> rects_;
     DeviceArray<int> tile_counts_;
-    DeviceArray<int> cull_counts_;  // exact-culling record counts per Gaussian
-    DeviceArray<uint4> cull_spans_;  // and the kept column intervals behind them
+    // Exact culling: the kept column intervals per Gaussian, then the record counts.
+    DeviceArray<uint4> cull_spans_;
+    int* CullCounts() const { return reinterpret_cast<int*>(cull_spans_.get() + gaussian_capacity_); }
     DeviceArray<uint32_t> depth_keys_[2];
     DeviceArray<uint32_t> depth_ids_[2];
     DeviceArray<int> record_start_;
     mutable DeviceArray<int> record_offsets_;
     mutable bool record_offsets_valid_ = false;
+    // Tile offsets (one more than tiles), then the tiles' bounds: one allocation, as a
+    // new renderer's first frame is bound by them.
     DeviceArray<int64_t> tile_offsets_;
+    int* TileBounds() const { return reinterpret_cast<int*>(tile_offsets_.get() + tile_capacity_ + 1); }
     DeviceArray<uint32_t> tile_keys_[2];
     DeviceArray<uint32_t> record_ids_[2];
     uint32_t* sorted_ids_ = nullptr;
     DeviceArray<int> contributors_;
     DeviceArray<uint32_t> record_warps_;
-    DeviceArray<int> tile_bounds_;
     mutable std::atomic<bool> keep_checkpoints_{false};
     mutable DeviceArray<float4> checkpoints_;
     int checkpoint_tiles_ = 0;  // of the last frame, 0 where it kept none

@@ -1,7 +1,8 @@
 """The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
 capture go on where there is none, without asking for it again; the buffer stays where
 it is for frames that need no more room; a frame's own buffers come before it; and a
-renderer whose frames no backward pass reads has none.
+renderer whose frames no backward pass reads has none. A first frame, which is bound by its
+allocations, takes no more of them than one per buffer.
 Allocations are counted and refused on the host, through the library's allocation hook."""
 import ctypes
 
@@ -163,3 +164,19 @@ def test_a_renderer_that_only_renders_keeps_no_checkpoints():
         segments = gradients(r, s, p, cam, target, image)
         assert seen.large() == 1
     assert close(whole, segments)
+
+
+@pytest.mark.parametrize("culled", [False, True])
+def test_a_first_frame_takes_one_allocation_per_buffer(culled):
+    """14 per-Gaussian and counter buffers (13 where no culled counts are kept), offsets with
+    bounds, contributors, five record buffers and two scratches."""
+    t = torch()
+    p, cam, _ = scene()
+    image = empty((H, W, 3), t.float32)
+    r = gsn.Renderer()
+    r.set_exact_culling(culled)
+    with Allocations() as seen:
+        assert r.set_record_capacity(CAPACITY) == 0
+        assert r.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
+        sync()
+        assert len(seen.sizes) == (23 if culled else 22)
