@@ -32,9 +32,12 @@
 //     rounded reciprocal;
 //   * where the frame has few tiles (the forward wrote checkpoints: T and the colour of
 //     every pixel after each kSegment records of its tile), a tile's list is cut into
-//     segments of kSegment records that run as independent warps, each starting from
-//     its checkpoint. A serial walk per tile left 11 warps per SM on 1,700 tiles of
-//     800 records, and the longest list decided the time;
+//     segments that run as independent warps, each starting from its checkpoint: kSegment
+//     records each where they are enough for the list, equal shares of whole kSegments
+//     where it is longer. A serial walk per tile left 11 warps per SM on 1,700 tiles of
+//     800 records, and the longest list decided the time; with the rest of a longer list
+//     on the last warp, 100k faint Gaussians on 250x180 took 14,080 us in the exact form
+//     (two warps per tile: 12,990) instead of 2,484;
 //   * a segment is a warp's whole work (a loop over segments made the compiler hold every
 //     pixel's inputs across it: 168 registers, or spills at 128, and 25 % more time).
 //   * the exact form skips the pairs of a quadrant that the record's ellipse does not
@@ -99,10 +102,17 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     // offsets are of different frames
     const int bound = static_cast<int>(
         min(static_cast<int64_t>(a.tile_bounds[tile]), a.tile_offsets[tile + 1] - begin));
-    // this warp's segment of it: kSegment records, the last warp's to the end
-    const int from = static_cast<int>(blockIdx.y) * kSegment;
+    // this warp's segment of it: kSegment records, or an equal share of whole kSegments
+    // where the list is longer than those. The reduction of equal values tells the compiler
+    // that they are equal: with `from` in a uniform register the kernel takes 116 registers
+    // instead of 126, with which the exact form is 3 % slower
+    const int span = kSegment * static_cast<int>(gridDim.y);
+    int length = kSegment;
+    if (bound > span) length = kSegment * ((bound + span - 1) / span);
+    length = __reduce_max_sync(0xffffffffu, length);
+    const int from = static_cast<int>(blockIdx.y) * length;
     if (from >= bound) return;
-    const int to = blockIdx.y + 1 == gridDim.y ? bound : min(bound, from + kSegment);
+    const int to = min(bound, from + length);
     const int tx = tile % a.cam.tile_count_x, ty = tile / a.cam.tile_count_x;
     using Layout = PairLayout<kFast>;
     const int x0 = tx * kTile + Layout::lane_x(lane), y0 = ty * kTile + Layout::lane_y(lane);
@@ -311,8 +321,9 @@ int launch_raster_backward(const RasterBackwardArgs& a, cudaStream_t stream) {
     if (!a.contributors || !a.tile_bounds || !a.record_warps || (reinterpret_cast<uintptr_t>(a.grad_out) & 15) != 0)
         return GSN_ERR_INVALID_ARGUMENT;
     // warps per tile: enough to fill the GPU (one whose segment lies past the tile's
-    // bound leaves at once); the last takes what is left of a longer list
-    const int64_t parts = a.checkpoints ? std::min<int64_t>(16, std::max<int64_t>(2, kSegmentWarps / tiles)) : 1;
+    // bound leaves at once), at least four at kCheckpointTiles
+    static_assert(kSegmentWarps / kCheckpointTiles >= 2, "a frame with checkpoints has segments");
+    const int64_t parts = a.checkpoints ? std::min<int64_t>(16, kSegmentWarps / tiles) : 1;
     const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(parts));
     if (a.fast) launch_step(raster_backward_kernel<true>, grid, 32, 0, stream, a);
     else launch_step(raster_backward_kernel<false>, grid, 32, 0, stream, a);

@@ -11,7 +11,7 @@ constexpr int kRasterBatch = 128;  // records the forward stages at a time
 // after each kSegment records of its tile, so that the backward pass can run the
 // segments of a long list side by side.
 constexpr int kSegment = 128;      // a batch of the forward pass
-constexpr int kSegmentWarps = 16384;  // warps a segmented launch aims at (148 SMs x 16 resident x 7)
+constexpr int kSegmentWarps = 16384;  // warps a segmented launch aims at (7 times 148 SMs x 16 resident, about)
 static_assert(kSegment == kRasterBatch, "checkpoints are written between batches");
 
 // Where the checkpoint before record `at` (a multiple of kSegment) of a tile's list

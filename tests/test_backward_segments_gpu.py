@@ -1,6 +1,6 @@
 """The backward blend on frames of few tiles, where a tile's list is cut into segments
 that start from the forward pass's checkpoints: screen-space gradients of lists from a
-handful of records to more than sixteen segments (the last warp takes the rest) against
+handful of records to more than sixteen strides (the warps share them evenly) against
 a float64 replay of the renderer's own lists, in both arithmetic forms, on ragged
 frames, and the same frame just above and below the tile count that switches it on."""
 import numpy as np
