@@ -36,9 +36,12 @@ constexpr int kSortChunk = kSortThreads * kSortItems;  // 3072 keys per block
 // 62.5 -> 52.2 at 600k, but 57.4 -> 64.3 at 800k and 72.7 -> 70.7 at 1M.
 constexpr int kMidItems = 4;
 constexpr int kMidCount = 512 * kSortThreads * kMidItems;
-// Up to kSmallCount keys one block does the whole sort in shared memory.
+// Up to kSmallCount keys one block does the whole sort in shared memory: 5,120 pairs take
+// 32.0 us on 32 bits, 17.0 on 13 and 11.2 on 8, the passes above 32.2, 18.4 and 12.0;
+// one block's 32.0, 17.0, 11.2 grow to 36.8, 19.1, 12.6 at 6,144 pairs and to 45.7, 22.8,
+// 15.2 at 8,192, those of the passes hardly.
 constexpr int kSmallThreads = 1024;
-constexpr int kSmallItems = 8;
+constexpr int kSmallItems = 5;
 constexpr int kSmallCount = kSmallThreads * kSmallItems;
 constexpr int kBins = 256;
 // Each pass's digit totals are kept as kTotalCopies partial copies, one 1 KB row
@@ -304,8 +307,8 @@ __global__ void radix_kept(const uint32_t* __restrict__ digit_total, int* __rest
 
 // The whole sort of at most kSmallCount pairs in one block: the same passes, digits
 // and stable ranking, with the pairs in shared memory between them. Three launches per
-// pass cost 15 us however few the keys are: 62 us for the 32-bit sort of 4,096 keys,
-// which takes 25 us here.
+// pass cost 10 us however few the keys are: 40 us for the 32-bit sort of 4,096 keys,
+// which takes 28 us here, and 37 us for 100 keys, which take 14.
 struct SmallSmem {
     uint32_t keys[kSmallCount], vals[kSmallCount];
     uint16_t counts[kSmallThreads / 32][kBins];  // a warp's keys per digit, then where its first goes

@@ -45,11 +45,11 @@ def test_sort_pairs_matches_stable_sort(n, bits):
     assert np.array_equal(k, ek) and np.array_equal(v, ev)
 
 
-@pytest.mark.parametrize("n", [1023, 1025, 8191, 8192, 8193, 262_144, 524_287, 524_288, 524_289])
+@pytest.mark.parametrize("n", [1023, 1025, 5119, 5120, 5121, 8191, 8192, 8193, 262_144, 524_287, 524_288, 524_289])
 @pytest.mark.parametrize("bits", [(0, 30), (3, 9), (8, 32)])
 @pytest.mark.parametrize("keys_of", ["uniform", "constant", "top"])
 def test_sort_pairs_at_the_edges_of_its_three_forms(n, bits, keys_of):
-    """One block up to 8,192 pairs, 4 keys per thread up to 524,288, 12 above: odd and
+    """One block up to 5,120 pairs, 4 keys per thread up to 524,288, 12 above: odd and
     even pass counts (results in either buffer), one digit holding every key, and the
     key that a dropping sort leaves out, which a plain sort keeps."""
     rng = np.random.default_rng(n + bits[0])
