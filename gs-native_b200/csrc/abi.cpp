@@ -137,7 +137,7 @@ int gsn_sort_pairs(uint32_t* keys, uint32_t* values, uint32_t* keys_alt, uint32_
     if (!keys || !values || !keys_alt || !values_alt || !workspace ||
         workspace_bytes < gsn::radix_sort_scratch_bytes(count))
         return GSN_ERR_INVALID_ARGUMENT;
-    gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(workspace, count);
+    gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(workspace);
     bool alt = false;
     int status = gsn::launch_radix_sort(keys, values, keys_alt, values_alt, false, count, nullptr, begin_bit, end_bit,
                                         scratch, &alt, AsStream(stream));

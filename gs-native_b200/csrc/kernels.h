@@ -78,12 +78,11 @@ int launch_project_tiled(const float* params, int n, const gsn_camera& cam, int 
 // grid is sized for `max_count` and every kernel reads the actual count from
 // device memory, so no host sync is needed.
 struct RadixSortScratch {
-    uint32_t* block_hist;   // [256 * max_blocks]
+    uint32_t* block_hist;   // [256][blocks of the sort]
     uint32_t* digit_total;  // [passes][16 partial copies][256]
-    size_t max_blocks;
 };
 size_t radix_sort_scratch_bytes(int max_count);
-RadixSortScratch radix_sort_scratch(void* base, int max_count);
+RadixSortScratch radix_sort_scratch(void* base);
 int launch_radix_sort(uint32_t* keys, uint32_t* values, uint32_t* keys_alt, uint32_t* values_alt,
                       bool identity_values, int max_count, const int* count_device, int begin_bit,
                       int end_bit, const RadixSortScratch& scratch, bool* result_in_alt,

@@ -420,7 +420,7 @@ int launch_knn3(const float* points, int n, float* mean_dist2, int* neighbors, v
     launch_step(curve_kernel, grid_for(n), kThreads, 0, s, points, n, bounds, keys);
     int launches = 2;
     bool alt = false;
-    RadixSortScratch scratch = radix_sort_scratch(w + L.sort, n);
+    RadixSortScratch scratch = radix_sort_scratch(w + L.sort);
     int st = launch_radix_sort(keys, ids, keys_alt, ids_alt, true, n, nullptr, 0, 30, scratch, &alt, s);
     if (st != GSN_OK) return st;
     const uint32_t* order = alt ? ids_alt : ids;

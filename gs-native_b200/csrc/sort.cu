@@ -112,7 +112,8 @@ __device__ __forceinline__ uint32_t digit_sum(const uint32_t* __restrict__ digit
 
 // One block per digit: exclusive scan of that digit's per-block counts, offset by
 // the number of keys with a smaller digit.
-__global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int n_host, int chunk,
+template <int kItems>
+__global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int n_host,
                                                            uint32_t* __restrict__ block_hist,
                                                            size_t hist_stride,
                                                            const uint32_t* __restrict__ digit_total) {
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scan(const int* n_dev, int
     __shared__ uint32_t warp_sums[kSortWarps];
     __shared__ uint32_t carry;
     const int n = load_count(n_dev, n_host);
-    const int blocks = ceil_div(n, chunk);
+    const int blocks = ceil_div(n, kItems * kSortThreads);
     const int d = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // base = sum of totals of smaller digits
@@ -706,9 +707,8 @@ size_t radix_sort_scratch_bytes(int max_count) {
     return radix_sort_scratch_words(max_count) * sizeof(uint32_t) + 256;
 }
 
-RadixSortScratch radix_sort_scratch(void* base, int max_count) {
+RadixSortScratch radix_sort_scratch(void* base) {
     RadixSortScratch s;
-    s.max_blocks = radix_sort_max_blocks(max_count);
     s.digit_total = static_cast<uint32_t*>(base);
     s.block_hist = s.digit_total + kDigitTotalWords * 4;
     return s;
@@ -734,17 +734,18 @@ static void radix_pass(uint32_t* kin, uint32_t* vin, uint32_t* kout, uint32_t* v
                        const int* count, int max_count, int bit, int digit_bits, uint32_t* totals,
                        const RadixSortScratch& scratch, cudaStream_t stream) {
     const int blocks = ceil_div(max_count, kItems * kSortThreads);
+    const size_t stride = static_cast<size_t>(blocks);  // of a digit's row of block counts
     const uint32_t mask = (1u << digit_bits) - 1u;
     auto up = drop ? radix_upsweep<true, kItems> : radix_upsweep<false, kItems>;
     launch_step(up, blocks, kSortThreads, 0, stream, kin, count, max_count, bit, mask, scratch.block_hist,
-                scratch.max_blocks, totals);
-    launch_step(radix_scan, 1 << digit_bits, kSortThreads, 0, stream, count, max_count, kItems * kSortThreads,
-                scratch.block_hist, scratch.max_blocks, totals);
+                stride, totals);
+    launch_step(radix_scan<kItems>, 1 << digit_bits, kSortThreads, 0, stream, count, max_count, scratch.block_hist,
+                stride, totals);
     auto down = identity ? (drop ? radix_downsweep<true, true, kItems> : radix_downsweep<true, false, kItems>)
                          : (drop ? radix_downsweep<false, true, kItems> : radix_downsweep<false, false, kItems>);
     const uint32_t* values = identity ? nullptr : vin;
     launch_step(down, blocks, kSortThreads, 0, stream, kin, values, kout, vout, count, max_count, bit, mask,
-                digit_bits, scratch.block_hist, scratch.max_blocks);
+                digit_bits, scratch.block_hist, stride);
 }
 
 static int radix_sort_impl(uint32_t* keys, uint32_t* values, uint32_t* keys_alt, uint32_t* values_alt,
@@ -852,7 +853,7 @@ int launch_radix_sort_noalloc(uint32_t* keys, uint32_t* values, uint32_t* keys_a
     // the layout for `count` pairs is a prefix of the array; the digit totals
     // are cleared by launch_radix_sort and every histogram word is written
     // before it is read, so nothing left by an earlier call is used
-    RadixSortScratch scratch = radix_sort_scratch(base, count);
+    RadixSortScratch scratch = radix_sort_scratch(base);
     return launch_radix_sort(keys, values, keys_alt, values_alt, false, count, nullptr, begin_bit, end_bit, scratch,
                              result_in_alt, stream);
 }

@@ -117,7 +117,7 @@ bool MultiViewRenderer::Prepare(View& v, const GaussianBuffers& g, const CameraP
         GSN_OK)
         return false;
     if (config_.key_bits == 32) {
-        gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(v.sort_scratch.get(), static_cast<int>(v.sort_scratch_count));
+        gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(v.sort_scratch.get());
         bool alt = false;
         if (gsn::launch_radix_sort(v.depth_keys[0].get(), v.depth_ids[0].get(), v.depth_keys[1].get(),
                                    v.depth_ids[1].get(), true, n, nullptr, 0, 32, scratch, &alt, stream) != GSN_OK)
@@ -141,7 +141,7 @@ bool MultiViewRenderer::Order(View& v, int n, cudaStream_t stream) {
         v.record_capacity = grow;
     }
     if (!SortScratch(v.sort_scratch, v.sort_scratch_count, std::max<int64_t>(r, n))) return false;
-    gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(v.sort_scratch.get(), static_cast<int>(v.sort_scratch_count));
+    gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(v.sort_scratch.get());
     const int records = static_cast<int>(r);
     bool alt = false;
     if (config_.key_bits == 32) {

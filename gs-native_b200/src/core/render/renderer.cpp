@@ -149,7 +149,6 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     sh_degree = std::clamp(sh_degree, 0, 3);
     const size_t pixels = static_cast<size_t>(camera.width_) * camera.height_;
     if (!ReserveAtAnyRate([&] { return ReserveFrame(count, tile_count, pixels); })) return false;
-    const int sort_max = static_cast<int>(std::max<int64_t>(count, record_capacity_));
     if (!host_records_ && cudaMallocHost(&host_records_, sizeof(int)) != cudaSuccess) {
         host_records_ = nullptr;
         return false;
@@ -171,7 +170,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
         gsn::stage_mark(s, gsn::kStageProject);
         if (gsn::launch_project(gaussians.gaussians_, count, cam, device_camera_, sh_degree, bf16_sh_, po, s) != GSN_OK) return false;
         gsn::stage_mark(s, gsn::kStageDepthSort);
-        gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(sort_scratch_.get(), sort_max);
+        gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(sort_scratch_.get());
         bool in_alt = false;
         // culled Gaussians (depth key 0xFFFFFFFF) leave the sort in its first
         // pass: the later passes, the record scan and the emission see only the
@@ -234,7 +233,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
                                            record_capacity_, overflow, s);
         if (emitted != GSN_OK) return false;
         const int max_records = fixed_capacity_ ? static_cast<int>(record_capacity_) : static_cast<int>(records);
-        scratch = gsn::radix_sort_scratch(sort_scratch_.get(), static_cast<int>(sort_scratch_count_));
+        scratch = gsn::radix_sort_scratch(sort_scratch_.get());
         in_alt = false;
         gsn::stage_mark(s, gsn::kStageTileSort);
         if (max_records > 0 &&

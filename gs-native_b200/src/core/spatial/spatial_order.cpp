@@ -23,7 +23,7 @@ const uint32_t* SpatialOrder::ComputeIn(unsigned char* work, const float* params
     auto* bounds = reinterpret_cast<uint32_t*>(work + 4 * array);
     if (gsn::launch_morton_keys(params, count, bounds, keys[0], stream) != GSN_OK) return nullptr;
     bool in_alt = false;
-    const gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(work + 4 * array + 256, count);
+    const gsn::RadixSortScratch scratch = gsn::radix_sort_scratch(work + 4 * array + 256);
     if (gsn::launch_radix_sort(keys[0], ids[0], keys[1], ids[1], true, count, nullptr, 0, 30, scratch, &in_alt,
                                stream) != GSN_OK)
         return nullptr;
