@@ -16,7 +16,6 @@
 #include "common.cuh"
 #include "kernels.h"
 
-#include <atomic>
 #include <mutex>
 
 namespace gsn {
@@ -714,20 +713,6 @@ RadixSortScratch radix_sort_scratch(void* base) {
     return s;
 }
 
-// Raises the small sort's dynamic shared-memory limit, once per device.
-static int configure_small() {
-    static std::atomic<bool> configured[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return GSN_ERR_CUDA;
-    if (!configured[device].load()) {
-        if (cudaFuncSetAttribute(radix_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(SmallSmem))) != cudaSuccess)
-            return GSN_ERR_CUDA;
-        configured[device].store(true);
-    }
-    return GSN_OK;
-}
-
 // One pass of the general sort with kItems keys per thread.
 template <int kItems>
 static void radix_pass(uint32_t* kin, uint32_t* vin, uint32_t* kout, uint32_t* vout, bool identity, bool drop,
@@ -758,8 +743,10 @@ static int radix_sort_impl(uint32_t* keys, uint32_t* values, uint32_t* keys_alt,
     if (passes > 4 || !keys || !keys_alt || !values || !values_alt) return GSN_ERR_INVALID_ARGUMENT;
     *result_in_alt = (passes % 2) == 1;
     if (max_count <= kSmallCount) {
-        const int st = configure_small();
-        if (st != GSN_OK) return st;
+        // a context's own setting, so made with every launch
+        if (cudaFuncSetAttribute(radix_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(SmallSmem))) != cudaSuccess)
+            return GSN_ERR_CUDA;
         // all inputs are read before the first output is written, so the pairs may be
         // sorted in place
         launch_step(radix_small, 1, kSmallThreads, sizeof(SmallSmem), stream, keys, values,
