@@ -18,9 +18,9 @@ cudaError_t DeviceAlloc(void** ptr, size_t bytes) {
     if (fn) return fn(ptr, bytes);
     cudaError_t e = cudaMalloc(ptr, bytes);
     if (e == cudaErrorMemoryAllocation) {
-        // what the scratch pools keep may be what is missing
+        // what the scratch pool keeps may be what is missing
         cudaGetLastError();
-        ReleaseStreamPools();
+        ReleaseStreamPool();
         e = cudaMalloc(ptr, bytes);
     }
     return e;

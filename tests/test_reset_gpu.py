@@ -18,6 +18,8 @@ import gsn
 n = 3000
 rng = np.random.default_rng(1)
 keys = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32)
+params = rng.normal(size=(58, n)).astype(np.float32)
+image, target = rng.random((48, 64, 3)).astype(np.float32), np.full((48, 64, 3), 70, np.uint8)
 
 
 def upload(array):
@@ -37,6 +39,19 @@ def sort():
     return out.tobytes()
 
 
+def order():
+    perm = upload(keys)
+    gsn.spatial_permutation(upload(params), n, perm)
+    out = np.zeros(n, np.uint32)
+    gsn.memcpy(out.ctypes.data, perm, out.nbytes)
+    assert np.array_equal(np.sort(out), np.arange(n))
+    return out.tobytes()
+
+
+def evaluate():
+    return gsn.eval_metrics(upload(image), upload(target), 64, 48)
+
+
 runtime = ctypes.CDLL("/usr/local/cuda/lib64/libcudart.so")
 first = {call}()
 for _ in range(2):
@@ -45,7 +60,7 @@ for _ in range(2):
 """
 
 
-@pytest.mark.parametrize("call", ["sort"])
+@pytest.mark.parametrize("call", ["sort", "order", "evaluate"])
 def test_stateless_calls_answer_after_a_reset(call):
     program = PROGRAM.format(package=ROOT + "/gs-native_b200", call=call)
     done = subprocess.run([sys.executable, "-c", program], capture_output=True, text=True, timeout=120)
