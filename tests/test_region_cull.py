@@ -1,8 +1,8 @@
-"""CPU check of the blend kernels' region test (raster_common.cuh cull_limit and
-region_hit) restated in float32: a record it drops for a rectangle of pixels has, in
-the kernels' own float32 arithmetic, alpha below 1/255 at each of them. Conics up to
-the condition number at which culling is switched off, means inside, beside and far
-from the rectangle, opacities down to the threshold."""
+"""CPU check of the formula of the blend kernels' region test (raster_common.cuh cull_limit
+and region_hit), restated in float32 with exact divides: a record it drops for a rectangle
+of pixels has alpha below 1/255 at each of them. Conics up to the condition number at which
+culling is switched off, means inside, beside and far from the rectangle, opacities down to
+the threshold. The kernels' own arithmetic is checked in test_region_cull_gpu.py."""
 import numpy as np
 import pytest
 
