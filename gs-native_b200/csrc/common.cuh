@@ -88,6 +88,14 @@ inline void launch_step(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, si
     cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
+// Element-wise atomic add of four floats at a 16-byte aligned global address
+// (PTX red.global.add with a .v4.f32 vector, sm_90 and later).
+__device__ __forceinline__ void red_add_v4(float* address, float4 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(address), "f"(v.x), "f"(v.y), "f"(v.z),
+                 "f"(v.w)
+                 : "memory");
+}
+
 // ---------------------------------------------------------------- layouts
 // Parameter block layouts. The plain form uses the reference's 58 fp32 rows of
 // stride N. The precision form keeps the 10 geometry rows (position, log-scale,

@@ -120,8 +120,12 @@ int launch_emit_records(const uint32_t* sorted_ids, const int* record_start, con
                         int64_t capacity, int* overflow, cudaStream_t stream);
 
 // Both emitters run resident blocks over the visible Gaussians (the host does not know
-// their number): at most kEmitBlocks of 256 threads.
+// their number): at most kEmitBlocks of 256 threads, kEmitLanes of them per Gaussian. With
+// 4 lanes the few records a lane writes at a time left half-written sectors and idle warps
+// (plain 75 -> 68 us and culled 75 -> 67 us at 1.2M Gaussians, culled 39 -> 24 us on 30k
+// large ones, 172 -> 149 us at 3.0M, where 4 lanes take 119).
 constexpr int kEmitBlocks = 148 * 8;
+constexpr int kEmitLanes = 8;
 int emit_blocks(int lanes, int n);
 
 // Exact tile culling (project.cu): with ProjectOutputs::cull_counts set, the
@@ -153,10 +157,10 @@ struct RasterForwardArgs {
     int* contributors;             // [P] optional: records consumed before the pixel finished
     // optional: two bit planes of record_words words (plane w at record_warps +
     // w * record_words, cleared by the caller); bit r of plane w is set when a
-    // pixel of warp w's strip took record r
+    // pixel of rows 8w..8w+7 of the tile took record r
     uint32_t* record_warps;
     int64_t record_words;
-    bool fast;                     // fast power / exp arithmetic (see raster_common.cuh Power)
+    bool fast;                     // fast power / exp arithmetic (see raster_common.cuh fast_record)
     int* tile_bounds;              // [T] optional: the largest contributor count of the tile
     // optional: checkpoint_blocks(records, tiles) blocks of 256 pixels (T, r, g, b), the
     // state of every pixel after each 128 records of its tile
@@ -168,11 +172,13 @@ struct RasterForwardArgs {
 };
 int launch_raster_forward(const RasterForwardArgs& a, cudaStream_t stream);
 
-// Frames of at most kCheckpointTiles tiles keep checkpoints: the backward blend took
-// 365 instead of 412 us on 2,170 tiles (30k large Gaussians) and 260 instead of 361 us
-// on 1,700 (100k). On 6,700 tiles one warp per tile fills the GPU: the 11 of 595 us that
-// segments save there do not pay for a 32 bytes per record larger workspace and the
-// forward pass's writes.
+// Frames of at most kCheckpointTiles tiles keep checkpoints. Scenes of 180 Gaussians per
+// tile, backward blend with and without them, exact form (fast form): 259 and 322 us (192,
+// 224) on 1,700 tiles, 361 and 471 (243, 273) on 3,024, 444 and 507 (288, 311) on 4,096, 483
+// and 552 (293, 309) on 5,355, 588 and 598 (325, 341) on 6,700; the forward pass's writes
+// do not show. A step gains 5 to 9 % on 1,700 tiles, 2 to 5 % on 4,096 and 0.4 to 1.4 % on
+// 6,700, where one warp per tile fills the GPU, for a workspace of 32 bytes per record
+// that grows with the frame: the line lies where the gain no longer pays for that.
 constexpr int kCheckpointTiles = 4096;
 size_t checkpoint_blocks(int64_t records, int tiles);
 

@@ -218,13 +218,6 @@ __global__ void __launch_bounds__(kMlpThreads, 2) mlp_infer_kernel(const float* 
     }
 }
 
-// Element-wise atomic add of four floats (PTX red.global.add.v4.f32, sm_90 and later).
-__device__ __forceinline__ void red_add_v4(float* address, float4 v) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(address), "f"(v.x), "f"(v.y), "f"(v.z),
-                 "f"(v.w)
-                 : "memory");
-}
-
 struct TrainSmem {
     Weights w;
     float w2_out[kHid * kHid];  // W2 output-major

@@ -113,7 +113,7 @@ __device__ __forceinline__ void blend_tile(const MultiView& v, int tile, float4*
                 for (int p = 0; p < P; ++p) {
                     const float pw = power.at(head.y - fy[p]);
                     const bool act = !done[p] && !(pw > 0.0f) && !(pw < tail.y);
-                    const float alpha = fminf(kAlphaMax, gaussian_weight<false>(q.w, pw));
+                    const float alpha = fminf(kAlphaMax, gaussian_weight(q.w, pw));
                     bool take = act && !(alpha < kAlphaMin);
                     const float nextT = T[p] * (1.0f - alpha);
                     const bool stop = take && nextT < kTransmittanceMin;

@@ -46,9 +46,9 @@ __device__ __forceinline__ void sh_basis(float x, float y, float z, float b[16])
 // alpha = o * exp(-q/2) >= 1/255, i.e. inside the ellipse q(d) <= 2 ln(255 o)
 // (q(d) = A dx^2 + 2 B dx dy + C dy^2, conic (A, B, C), d = pixel - mean). The
 // reference emits every tile of the 3-sigma rectangle; the culled form emits only
-// the tiles whose pixel-centre rectangle meets that ellipse, widened as the blend
-// kernels' alpha box is (2 % + 0.05 on Q plus a condition-number term, and a
-// pixel pad), so a dropped record is one the per-pixel test rejects at every
+// the tiles whose pixel-centre rectangle meets that ellipse, widened as in the blend
+// kernels' region test (2 % + 0.05 on Q plus a condition-number term) and by a
+// pixel pad, so a dropped record is one the per-pixel test rejects at every
 // pixel of its tile: images, transmittance and gradients are unchanged.
 //
 // Per tile row the reachable columns form one interval: the ellipse's x-extent
@@ -164,12 +164,6 @@ __device__ __forceinline__ int cull_count(float2 mean, float4 q, int4 rect, uint
     }
     return total;
 }
-
-// 8 lanes per Gaussian here and in emit_records (sort.cu), in resident blocks over the
-// visible ones: with 4 lanes the few records a lane writes at a time left half-written
-// sectors and idle warps (plain 75 -> 68 us and culled 75 -> 67 us at 1.2M Gaussians,
-// culled 39 -> 24 us on 30k large ones, 172 -> 149 us at 3.0M, where 4 lanes take 119).
-constexpr int kEmitLanes = 8;
 
 // Records of the culled counts in depth order. kEmitLanes lanes serve a
 // Gaussian. Where its intervals were kept, each lane writes every kEmitLanes-th record,

@@ -75,14 +75,6 @@ struct PairLayout {
 };
 constexpr int kBatch = 32;      // records staged per batch (one per lane)
 
-// Element-wise atomic add of four floats at a 16-byte aligned global address
-// (PTX red.global.add with a .v4.f32 vector, sm_90 and later).
-__device__ __forceinline__ void red_add_v4(float* address, float4 v) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(address), "f"(v.x), "f"(v.y), "f"(v.z),
-                 "f"(v.w)
-                 : "memory");
-}
-
 template <bool kFast>
 __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardArgs a) {
     pdl_begin();
@@ -225,8 +217,8 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
                 } else {
                     const Power power(q, dx);
                     const float pw0 = power.at(dy.x), pw1 = power.at(dy.y);
-                    const float raw0 = gaussian_weight<false>(q.w, pw0);
-                    const float raw1 = gaussian_weight<false>(q.w, pw1);
+                    const float raw0 = gaussian_weight(q.w, pw0);
+                    const float raw1 = gaussian_weight(q.w, pw1);
                     const bool take0 = idx < limit[2 * h] && !(pw0 > 0.0f) && !(pw0 < aux.x) &&
                                        !(raw0 < kAlphaMin);
                     const bool take1 = idx < limit[2 * h + 1] && !(pw1 > 0.0f) && !(pw1 < aux.x) &&

@@ -95,12 +95,8 @@ struct Power {
     }
 };
 
-// o * e^power: the reference's expf in the exact form, the hardware exp2
-// approximation (__expf) in the fast form.
-template <bool kFast>
-__device__ __forceinline__ float gaussian_weight(float opacity, float power) {
-    return kFast ? opacity * __expf(power) : opacity * expf(power);
-}
+// o * e^power of the exact form, with the reference's expf.
+__device__ __forceinline__ float gaussian_weight(float opacity, float power) { return opacity * expf(power); }
 
 // 1 / x for x in [0.01, 1] (one minus a clamped alpha): the correctly rounded
 // reciprocal in the exact form, the single hardware approximation (PTX

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
                     for (int p = 0; p < kForwardPix; ++p) {
                         const float pw = power.at(head.y - fy[p]);
                         const bool act = !done[p] && !(pw > 0.0f) && !(pw < lim);
-                        const float alpha = fminf(kAlphaMax, gaussian_weight<false>(q.w, pw));
+                        const float alpha = fminf(kAlphaMax, gaussian_weight(q.w, pw));
                         bool take = act && !(alpha < kAlphaMin);
                         const float nextT = T[p] * (1.0f - alpha);
                         const bool stop = take && nextT < kTransmittanceMin;

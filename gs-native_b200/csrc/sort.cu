@@ -579,8 +579,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
 }
 
 // ---------------------------------------------------------------- records
-constexpr int kEmitLanes = 8;
-
 // kEmitLanes lanes per Gaussian walk its tile rectangle row-major (stepping the column
 // instead of dividing by the width); the records of one
 // Gaussian are contiguous and in the same order as the reference writes them.
