@@ -98,6 +98,7 @@ int main(int argc, char** argv) {
         buffers.gaussians_ = device_params;
         buffers.gaussian_count_ = count;
         gs_native::Renderer renderer;
+        renderer.ExpectNoBackward();
         const float background[3] = {0.0f, 0.0f, 0.0f};
         std::vector<float> image;
         double sum = 0;

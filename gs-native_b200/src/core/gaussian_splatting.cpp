@@ -93,6 +93,7 @@ bool GaussianSplatting::Initialize(const TrainingScene& scene, const TrainingOpt
     renderer_.SetExactCulling(options_.exact_culling);
     renderer_.SetFastBlend(options_.fast_blend);
     eval_renderer_.SetBf16Sh(options_.bf16_sh);
+    eval_renderer_.ExpectNoBackward();
     solver_.SetBf16Sh(options_.bf16_sh);
     if (options_.bf16_sh && options_.fp32_ssim) solver_.SetTensorCoreLoss(false);
     density_.SetBf16Sh(options_.bf16_sh);

@@ -42,14 +42,13 @@ bool Renderer::SetRecordCapacity(int64_t records) {
 
 bool Renderer::ReserveGaussians(int count) {
     size_t n = static_cast<size_t>(std::max(count, 1));
-    if (n <= gaussian_capacity_ && counters_.get()) return true;
+    if (n <= gaussian_capacity_ && record_start_.get()) return true;
     size_t grow = std::max(n, gaussian_capacity_ + gaussian_capacity_ / 4);
     bool ok = means_.Reserve(grow) && conic_opacities_.Reserve(grow) && colors_.Reserve(grow) &&
               depths_.Reserve(grow) && radii_.Reserve(grow) && rects_.Reserve(grow) &&
               tile_counts_.Reserve(grow) && depth_keys_[0].Reserve(grow) &&
               depth_keys_[1].Reserve(grow) &&
-              depth_ids_[0].Reserve(grow) && depth_ids_[1].Reserve(grow) && record_start_.Reserve(grow + 1) &&
-              counters_.Reserve(3);
+              depth_ids_[0].Reserve(grow) && depth_ids_[1].Reserve(grow) && record_start_.Reserve(grow + 1 + 3);
     if (!ok) return false;
     gaussian_capacity_ = grow;
     return true;
@@ -98,6 +97,11 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
     return !exact_culling_ || cull_spans_.Reserve(gaussian_capacity_ + (gaussian_capacity_ + 3) / 4);
 }
 
+bool Renderer::Capturing() const {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream_, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+}
+
 // Without checkpoints the backward pass walks whole lists, so a frame goes on where
 // there is no memory for them, and does not ask again for as much: every later frame
 // would pay for the failing call. Nothing is allocated while the stream is captured,
@@ -105,13 +109,12 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
 // buffer moves only when tile_offsets_ or the record buffers do, so that a graph
 // captured over them outlives eager frames of other sizes.
 void Renderer::ReserveCheckpoints(int64_t tile_count) const {
-    if (!keep_checkpoints_.load() || tile_count > gsn::kCheckpointTiles) return;
+    if (tile_count > gsn::kCheckpointTiles) return;
     const int tiles = std::min(std::max(static_cast<int>(tile_count), GetTileCapacity()), gsn::kCheckpointTiles);
     const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tiles);
     if (blocks * kBlockPixels <= checkpoints_.capacity() || (checkpoint_refused_ && blocks >= checkpoint_refused_))
         return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream_, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+    if (Capturing()) return;
     if (!checkpoints_.Reserve(blocks * kBlockPixels)) {
         checkpoint_refused_ = blocks;
         cudaGetLastError();
@@ -120,7 +123,7 @@ void Renderer::ReserveCheckpoints(int64_t tile_count) const {
 
 // Reserves at once, so that one step is enough of a warm-up before a capture.
 void Renderer::KeepCheckpoints(int64_t tiles) const {
-    if (!keep_checkpoints_.exchange(true)) ReserveCheckpoints(tiles);
+    if (!backward_.exchange(true)) ReserveCheckpoints(tiles);
 }
 
 // The frame's own buffers come before the checkpoints. Not with a fixed capacity: a
@@ -157,7 +160,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
     last_count_ = count;
     const gsn_camera& cam = AsGsnCamera(camera);
     cudaStream_t s = stream_;
-    if (cudaMemsetAsync(counters_.get(), 0, 2 * sizeof(int), s) != cudaSuccess) return false;
+    if (cudaMemsetAsync(Counters(), 0, 2 * sizeof(int), s) != cudaSuccess) return false;
 
     int64_t records = 0;
     if (count > 0) {
@@ -175,7 +178,7 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
         // culled Gaussians (depth key 0xFFFFFFFF) leave the sort in its first
         // pass: the later passes, the record scan and the emission see only the
         // visible ones (their order - depth, then id - is unchanged)
-        int* visible = counters_.get() + 2;
+        int* visible = Counters() + 2;
         if (gsn::launch_radix_sort_dropping(depth_keys_[0].get(), depth_ids_[0].get(), depth_keys_[1].get(),
                                             depth_ids_[1].get(), true, count, nullptr, 0, fast_blend_ ? 24 : 32,
                                             scratch, &in_alt, visible, s) != GSN_OK)
@@ -189,8 +192,11 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
             cudaSuccess)
             return false;
     }
-    ReserveCheckpoints(tile_count);
-    return Blend(cam, background, image, tile_count);
+    if (backward_.load() || !rendered_) ReserveCheckpoints(tile_count);
+    else if (checkpoints_.get() && !Capturing()) checkpoints_.Reset();
+    if (!Blend(cam, background, image, tile_count)) return false;
+    rendered_ = true;
+    return true;
 }
 
 // Per-tile lists by emitting the records in depth order and stable-sorting
@@ -198,8 +204,8 @@ bool Renderer::Render(const GaussianBuffers& gaussians, const CameraParams& came
 bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int count, const CameraParams& camera,
                            int tile_count, int64_t* records_out) {
     cudaStream_t s = stream_;
-    int* record_count = counters_.get();
-    int* overflow = counters_.get() + 1;
+    int* record_count = Counters();
+    int* overflow = Counters() + 1;
     int64_t records = 0;
     gsn::RadixSortScratch scratch;
     bool in_alt = false;
@@ -255,7 +261,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 // The per-tile blend of the ordered records.
 bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
-    const bool checkpoints = keep_checkpoints_.load() && tile_count <= gsn::kCheckpointTiles &&
+    const bool checkpoints = (backward_.load() || !rendered_) && tile_count <= gsn::kCheckpointTiles &&
                              gsn::checkpoint_blocks(record_capacity_, tile_count) * kBlockPixels <= checkpoints_.capacity();
     checkpoint_tiles_ = checkpoints ? tile_count : 0;
     gsn::RasterForwardArgs ra;

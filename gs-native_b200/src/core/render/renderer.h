@@ -93,18 +93,20 @@ public:
     int64_t GetRecordWords() const { return record_words_; }
     // Per tile of the last frame, the largest contributor count of its pixels.
     const int* GetTileBounds() const { return TileBounds(); }
-    // A backward pass reads this renderer's frames: those after the call keep checkpoints
-    // (the solver calls it; before it a renderer, which may only ever render, holds none).
-    // `tiles`: of the last frame.
+    // A backward pass reads this renderer's frames (the solver says so): all after the call
+    // keep checkpoints. Without it only the first frame does, since a renderer whose first
+    // frame was not used so probably only renders. `tiles`: of the last frame.
     void KeepCheckpoints(int64_t tiles) const;
+    // No backward pass is expected: the first frame keeps no checkpoints either.
+    void ExpectNoBackward() { rendered_ = true; }
     // Per-pixel blend states inside long lists, kept for frames of few tiles: the
     // backward pass starts its segments from them. Null where the last frame kept none
     // or had another number of tiles.
     const float4* GetCheckpoints(int64_t tiles) const {
         return checkpoint_tiles_ == tiles ? checkpoints_.get() : nullptr;
     }
-    const int* GetRecordCountDevice() const { return counters_.get(); }
-    const int* GetOverflowFlag() const { return counters_.get() + 1; }
+    const int* GetRecordCountDevice() const { return Counters(); }
+    const int* GetOverflowFlag() const { return Counters() + 1; }
     int64_t GetRecordCapacity() const { return record_capacity_; }
     // Record count of the last Render() (valid in grow mode without a sync).
     int64_t GetLastRecordCount() const { return last_records_; }
@@ -118,6 +120,7 @@ private:
     bool ReserveFrame(int count, int tile_count, size_t pixels);
     // Room for a frame's checkpoints, where there is memory for them.
     void ReserveCheckpoints(int64_t tile_count) const;
+    bool Capturing() const;
     // reserve() again without the checkpoints, where it fails with them.
     template <typename Reserve>
     bool ReserveAtAnyRate(Reserve reserve);
@@ -151,7 +154,10 @@ private:
     int* CullCounts() const { return reinterpret_cast<int*>(cull_spans_.get() + gaussian_capacity_); }
     DeviceArray<uint32_t> depth_keys_[2];
     DeviceArray<uint32_t> depth_ids_[2];
+    // Record starts (one more than Gaussians), then the counters: record count, overflow
+    // flag, visible Gaussians.
     DeviceArray<int> record_start_;
+    int* Counters() const { return record_start_.get() + gaussian_capacity_ + 1; }
     mutable DeviceArray<int> record_offsets_;
     mutable bool record_offsets_valid_ = false;
     // Tile offsets (one more than tiles), then the tiles' bounds: one allocation, as a
@@ -163,7 +169,8 @@ private:
     uint32_t* sorted_ids_ = nullptr;
     DeviceArray<int> contributors_;
     DeviceArray<uint32_t> record_warps_;
-    mutable std::atomic<bool> keep_checkpoints_{false};
+    bool rendered_ = false;  // a frame has been rendered
+    mutable std::atomic<bool> backward_{false};  // a backward pass has read one
     mutable DeviceArray<float4> checkpoints_;
     int checkpoint_tiles_ = 0;  // of the last frame, 0 where it kept none
     mutable size_t checkpoint_refused_ = 0;  // blocks there was no memory for (0: none refused)
@@ -173,7 +180,6 @@ private:
     size_t sort_scratch_count_ = 0;
     mutable DeviceArray<unsigned char> scan_scratch_;
     mutable size_t scan_scratch_count_ = 0;
-    DeviceArray<int> counters_;  // [0] record count, [1] overflow flag, [2] visible Gaussians
     int* host_records_ = nullptr;  // pinned
 };
 

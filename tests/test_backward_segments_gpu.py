@@ -20,13 +20,12 @@ def frame(params, cam, target, fast):
     image = empty((cam.height, cam.width, 3), t.float32)
     r, s = gsn.Renderer(), gsn.Solver()
     r.set_fast_blend(fast)
-    for _ in range(2):  # checkpoints are kept from the first backward pass on
-        assert r.render(p.data_ptr(), n, cam, [0.1, 0.2, 0.3], image.data_ptr(), 0) == 0
-        gptr = s.image_gradients(cam, image.data_ptr(), tgt.data_ptr())
-        sync()
-        grad = host(gptr, np.float32, image.numel()).reshape(cam.height, cam.width, 3).astype(np.float64)
-        sptr = s.screen_gradients(cam, r, image.data_ptr(), p.data_ptr(), n)
-        sync()
+    assert r.render(p.data_ptr(), n, cam, [0.1, 0.2, 0.3], image.data_ptr(), 0) == 0
+    gptr = s.image_gradients(cam, image.data_ptr(), tgt.data_ptr())
+    sync()
+    grad = host(gptr, np.float32, image.numel()).reshape(cam.height, cam.width, 3).astype(np.float64)
+    sptr = s.screen_gradients(cam, r, image.data_ptr(), p.data_ptr(), n)
+    sync()
     b = r.buffers()
     records = int(b.record_count_host)
     return dict(screen=host(sptr, np.float32, 12 * n).reshape(n, 12), grad=grad,

@@ -1,9 +1,9 @@
 """The forward pass's checkpoints are optional memory: a frame, its gradients and a graph
 capture go on where there is none, without asking for it again; the buffer stays where
 it is for frames that need no more room; a frame's own buffers come before it; and a
-renderer whose frames no backward pass reads has none. A first frame, which is bound by its
-allocations, takes no more of them than one per buffer.
-Allocations are counted and refused on the host, through the library's allocation hook."""
+renderer whose first frame no backward pass reads gives it back. A first frame, which is
+bound by its allocations, takes no more of them than one per buffer. Allocations are
+counted and refused on the host, through the library's allocation hook."""
 import ctypes
 
 import numpy as np
@@ -153,23 +153,44 @@ def test_a_renderer_that_only_renders_keeps_no_checkpoints():
     p, cam, target = scene()
     image = empty((H, W, 3), t.float32)
     r, s = gsn.Renderer(), gsn.Solver()
+
+    def render():
+        assert r.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
+        sync()
+        return t.cuda.mem_get_info()[0]
+
     with Allocations() as seen:
         assert r.set_record_capacity(CAPACITY) == 0
-        for _ in range(3):
-            assert r.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
-        sync()
-        assert seen.large() == 0
-        whole = gradients(r, s, p, cam, target, image)
-        assert seen.large() == 1  # by the first backward pass, for the next frame
-        segments = gradients(r, s, p, cam, target, image)
+        first = render()
+        assert seen.large() == 1  # a first frame may be the first of a step
+        for _ in range(2):
+            assert render() - first >= LARGE  # it was not: given back
         assert seen.large() == 1
+        whole = gradients(r, s, p, cam, target, image)
+        assert seen.large() == 2  # by the backward pass, for the frames from now on
+        segments = gradients(r, s, p, cam, target, image)
+        assert render() < first + LARGE and seen.large() == 2
     assert close(whole, segments)
+
+
+def test_a_trainers_evaluation_keeps_no_checkpoints():
+    p, cam, target = scene()
+    rng = np.random.default_rng(6)
+    trainer = gsn.Trainer()
+    assert trainer.initialize([cam], [target.cpu().numpy()], rng.normal(0, 0.3, (200, 3)) + [0, 0, 3],
+                              rng.random((200, 3)), gsn.TrainingOptions.defaults()) == 0
+    image = empty((H, W, 3), torch().float32)
+    with Allocations() as seen:
+        assert trainer.render(cam, image.data_ptr()) == 0
+        sync()
+    assert seen.sizes  # the first evaluation makes its buffers; no whole blocks of checkpoints
+    assert not [size for size in seen.sizes if size % 4096 == 0 and size >= 4096 * cam.tiles]
 
 
 @pytest.mark.parametrize("culled", [False, True])
 def test_a_first_frame_takes_one_allocation_per_buffer(culled):
-    """14 per-Gaussian and counter buffers (13 where no culled counts are kept), offsets with
-    bounds, contributors, five record buffers and two scratches."""
+    """13 per-Gaussian buffers (12 where no culled counts are kept), offsets with bounds,
+    contributors, five record buffers, two scratches and the checkpoints."""
     t = torch()
     p, cam, _ = scene()
     image = empty((H, W, 3), t.float32)
