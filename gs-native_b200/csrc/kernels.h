@@ -162,7 +162,7 @@ struct RasterForwardArgs {
     int64_t record_words;
     bool fast;                     // fast power / exp arithmetic (see raster_common.cuh fast_record)
     int* tile_bounds;              // [T] optional: the largest contributor count of the tile
-    // optional: checkpoint_blocks(records, tiles) blocks of 256 pixels (T, r, g, b), the
+    // optional: checkpoint_blocks(records) blocks of 256 pixels (T, r, g, b), the
     // state of every pixel after each 128 records of its tile
     float4* checkpoints;
     // optional: adds the number of (pixel, record) pairs the blend took (the
@@ -180,7 +180,7 @@ int launch_raster_forward(const RasterForwardArgs& a, cudaStream_t stream);
 // 6,700, where one warp per tile fills the GPU, for a workspace of 32 bytes per record
 // that grows with the frame: the line lies where the gain no longer pays for that.
 constexpr int kCheckpointTiles = 4096;
-size_t checkpoint_blocks(int64_t records, int tiles);
+size_t checkpoint_blocks(int64_t records);
 
 // ---------------------------------------------------------------- loss
 // dL/dimage of 0.8 * L1 + 0.2 * (1 - SSIM) for an fp32 HWC image against a u8

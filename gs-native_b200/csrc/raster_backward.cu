@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(32, 16) raster_backward_kernel(RasterBackwardA
     float2 T2[kPairs], P2[kPairs], gI2[kPairs][3];
     int limit[2 * kPairs];
     const float4* checkpoint = nullptr;
-    if (from > 0) checkpoint = a.checkpoints + checkpoint_slot(begin, tile, from) * kTilePixels;
+    if (from > 0) checkpoint = a.checkpoints + checkpoint_slot(begin, from) * kTilePixels;
 #pragma unroll
     for (int p = 0; p < 2 * kPairs; ++p) {
         const int px = x0 + Layout::column(p >> 1), py = y0 + Layout::row(p >> 1) + Layout::kStep * (p & 1);

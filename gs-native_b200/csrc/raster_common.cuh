@@ -14,11 +14,12 @@ constexpr int kSegment = 128;      // a batch of the forward pass
 constexpr int kSegmentWarps = 16384;  // warps a segmented launch aims at (7 times 148 SMs x 16 resident, about)
 static_assert(kSegment == kRasterBatch, "checkpoints are written between batches");
 
-// Where the checkpoint before record `at` (a multiple of kSegment) of a tile's list
-// starts, in blocks of 256 pixels: floor sums keep the slots of different tiles apart,
-// and the last one is below records / kSegment + tiles.
-__device__ __forceinline__ int64_t checkpoint_slot(int64_t tile_begin, int tile, int at) {
-    return tile_begin / kSegment + tile + at / kSegment - 1;
+// Where the checkpoint before record `at` (a positive multiple of kSegment) of a tile's
+// list lies, in blocks of 256 pixels. Each stands for a record, of which a tile's next is
+// kSegment further on; the next tile begins behind all of them and starts with a stride
+// of its own, so no two share a slot, and the last one is below records / kSegment.
+__device__ __forceinline__ int64_t checkpoint_slot(int64_t tile_begin, int at) {
+    return tile_begin / kSegment + at / kSegment - 1;
 }
 
 // Which records can matter to a rectangle of pixels. With conic (A, B, C) and

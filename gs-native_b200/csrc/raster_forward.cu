@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
         for (int p = 0; p < kForwardPix; ++p) mine = mine && done[p];
         if (__syncthreads_and(mine)) break;
         if (a.checkpoints && base > begin) {
-            float4* state = a.checkpoints +
-                            checkpoint_slot(begin, tile, static_cast<int>(base - begin)) * kTilePixels;
+            float4* state =
+                a.checkpoints + checkpoint_slot(begin, static_cast<int>(base - begin)) * kTilePixels;
             const int in_tile = (8 * (warp >> 1) + (lane >> 3)) * kTile + 8 * (warp & 1) + (lane & 7);
 #pragma unroll
             for (int p = 0; p < kForwardPix; ++p)
@@ -267,9 +267,7 @@ __global__ void __launch_bounds__(kForwardThreads) raster_forward_kernel(RasterF
 
 }  // namespace
 
-size_t checkpoint_blocks(int64_t records, int tiles) {
-    return static_cast<size_t>(records) / kSegment + static_cast<size_t>(tiles);
-}
+size_t checkpoint_blocks(int64_t records) { return static_cast<size_t>(records) / kSegment; }
 
 int launch_raster_forward(const RasterForwardArgs& a, cudaStream_t stream) {
     int64_t tiles = static_cast<int64_t>(a.cam.tile_count_x) * a.cam.tile_count_y;

@@ -88,7 +88,8 @@ bool Renderer::ReserveFrame(int count, int tile_count, size_t pixels) {
         if (!contributors_.Reserve(pixels)) return false;
         pixel_capacity_ = pixels;
     }
-    if (!fixed_capacity_ && !ReserveRecords(std::max<int64_t>(record_capacity_, 1))) return false;
+    // with Gaussians in the frame the record buffers follow their count (OrderBySort)
+    if (!fixed_capacity_ && count == 0 && !ReserveRecords(std::max<int64_t>(record_capacity_, 1))) return false;
     if (!ReserveSort(std::max<int64_t>(count, record_capacity_))) return false;
     if (static_cast<size_t>(count) > scan_scratch_count_ || !scan_scratch_.get()) {
         if (!scan_scratch_.Reserve(gsn::scan_scratch_bytes(std::max(count, 1)))) return false;
@@ -105,13 +106,11 @@ bool Renderer::Capturing() const {
 // Without checkpoints the backward pass walks whole lists, so a frame goes on where
 // there is no memory for them, and does not ask again for as much: every later frame
 // would pay for the failing call. Nothing is allocated while the stream is captured,
-// where cudaMalloc would end the capture. Sized for the tiles reserved so far, the
-// buffer moves only when tile_offsets_ or the record buffers do, so that a graph
-// captured over them outlives eager frames of other sizes.
+// where cudaMalloc would end the capture. Sized by the record buffers, it moves only when
+// they do, so that a graph captured over them outlives eager frames of other sizes.
 void Renderer::ReserveCheckpoints(int64_t tile_count) const {
     if (tile_count > gsn::kCheckpointTiles) return;
-    const int tiles = std::min(std::max(static_cast<int>(tile_count), GetTileCapacity()), gsn::kCheckpointTiles);
-    const size_t blocks = gsn::checkpoint_blocks(record_capacity_, tiles);
+    const size_t blocks = gsn::checkpoint_blocks(record_capacity_);
     if (blocks * kBlockPixels <= checkpoints_.capacity() || (checkpoint_refused_ && blocks >= checkpoint_refused_))
         return;
     if (Capturing()) return;
@@ -262,7 +261,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
 bool Renderer::Blend(const gsn_camera& cam, const float* background, float* image, int tile_count) {
     cudaStream_t s = stream_;
     const bool checkpoints = (backward_.load() || !rendered_) && tile_count <= gsn::kCheckpointTiles &&
-                             gsn::checkpoint_blocks(record_capacity_, tile_count) * kBlockPixels <= checkpoints_.capacity();
+                             gsn::checkpoint_blocks(record_capacity_) * kBlockPixels <= checkpoints_.capacity();
     checkpoint_tiles_ = checkpoints ? tile_count : 0;
     gsn::RasterForwardArgs ra;
     ra.tile_ids = sorted_ids_;

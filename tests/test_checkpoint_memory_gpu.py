@@ -19,7 +19,7 @@ pytestmark = pytest.mark.gpu
 HOOK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t)
 CUDA_ERROR_MEMORY_ALLOCATION = 2
 W, H, COUNT, CAPACITY = 64, 48, 1500, 1 << 20
-# (CAPACITY / 128 + tiles) blocks of 256 float4: 32 MB; every other buffer here is below 5 MB
+# CAPACITY / 128 blocks of 256 float4: 32 MB; every other buffer here is below 5 MB
 LARGE = 16 << 20
 
 
@@ -183,21 +183,36 @@ def test_a_trainers_evaluation_keeps_no_checkpoints():
     with Allocations() as seen:
         assert trainer.render(cam, image.data_ptr()) == 0
         sync()
-    assert seen.sizes  # the first evaluation makes its buffers; no whole blocks of checkpoints
-    assert not [size for size in seen.sizes if size % 4096 == 0 and size >= 4096 * cam.tiles]
+    # the first evaluation makes its buffers; whole blocks of 4,096 bytes are checkpoints, or
+    # the contributors
+    assert [size for size in seen.sizes if size % 4096 == 0] == [4 * W * H]
 
 
 @pytest.mark.parametrize("culled", [False, True])
-def test_a_first_frame_takes_one_allocation_per_buffer(culled):
-    """13 per-Gaussian buffers (12 where no culled counts are kept), offsets with bounds,
-    contributors, five record buffers, two scratches and the checkpoints."""
+@pytest.mark.parametrize("capacity", [0, CAPACITY])
+def test_a_first_frame_takes_one_allocation_per_buffer(culled, capacity):
+    """12 per-Gaussian buffers (13 with culled counts), offsets with bounds, contributors, five
+    record buffers, two scratches (one again for the records in grow mode) and checkpoints."""
     t = torch()
     p, cam, _ = scene()
     image = empty((H, W, 3), t.float32)
     r = gsn.Renderer()
     r.set_exact_culling(culled)
     with Allocations() as seen:
-        assert r.set_record_capacity(CAPACITY) == 0
+        if capacity:
+            assert r.set_record_capacity(capacity) == 0
         assert r.render(p.data_ptr(), COUNT, cam, [0, 0, 0], image.data_ptr(), 0) == 0
         sync()
-        assert len(seen.sizes) == (23 if culled else 22)
+        assert len(seen.sizes) == 22 + (1 if culled else 0) + (0 if capacity else 1)
+
+
+def test_an_empty_first_frame_keeps_no_checkpoints():
+    t = torch()
+    _, cam, _ = scene()
+    image = empty((H, W, 3), t.float32)
+    r = gsn.Renderer()
+    with Allocations() as seen:
+        assert r.render(0, 0, cam, [0.25, 0.5, 0.75], image.data_ptr(), 0) == 0
+        sync()
+        assert len(seen.sizes) == 21
+    assert torch().equal(image, t.tensor([0.25, 0.5, 0.75], device="cuda").expand(H, W, 3))
