@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <climits>
 #include <mutex>
 
 namespace gsn {
@@ -467,7 +468,9 @@ __device__ __forceinline__ int block_exclusive_scan(int x, int* warp_sums, int* 
 // publishes its own. Status words hold the flag in the top two bits and the
 // value below. A word that stays unpublished for kScanPolls polls sets *error
 // and ends the walk; offsets then come out too small but never negative, and
-// every write stays inside the n + 1 outputs.
+// every write stays inside the n + 1 outputs. Sums beyond the range of int stay at its
+// largest value, since a wrapped record offset would lie in front of the record buffers
+// (a chunk's own sum, of 2,048 Gaussians' tile counts, is taken modulo 2^32).
 constexpr uint64_t kScanAggregate = 1ull << 62;
 constexpr uint64_t kScanInclusive = 2ull << 62;
 constexpr uint64_t kScanValue = (1ull << 62) - 1;
@@ -481,6 +484,10 @@ __device__ __forceinline__ unsigned long long load_scan_status(const unsigned lo
     unsigned long long value;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(value) : "l"(address) : "memory");
     return value;
+}
+
+__device__ __forceinline__ int scan_offset(long long sum) {
+    return static_cast<int>(min(sum, static_cast<long long>(INT_MAX)));
 }
 
 __device__ __forceinline__ long long warp_sum64(long long v) {
@@ -524,7 +531,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
     int run = block_exclusive_scan(sum, warp_sums, &total);
     if (threadIdx.x == 0) {
         store_scan_status(status + chunk, (chunk == 0 ? kScanInclusive : kScanAggregate) |
-                                              static_cast<unsigned long long>(total));
+                                              static_cast<uint32_t>(total));
         if (chunk == 0) s_excl = 0;
     }
     if (chunk > 0 && warp == 0) {
@@ -556,7 +563,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
             }
         }
         if (lane == 0) {
-            store_scan_status(status + chunk, kScanInclusive | static_cast<unsigned long long>(excl + total));
+            store_scan_status(status + chunk, kScanInclusive | static_cast<unsigned long long>(excl + static_cast<uint32_t>(total)));
             s_excl = excl;
         }
     }
@@ -564,7 +571,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
     const long long base = s_excl;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        tile[threadIdx.x * kScanItems + k] = static_cast<int>(base + run);
+        tile[threadIdx.x * kScanItems + k] = scan_offset(base + static_cast<uint32_t>(run));
         run += v[k];
     }
     __syncthreads();
@@ -575,7 +582,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_onepass(const int* in, cons
         if (i < n) out[i] = tile[j];
     }
     // the chunk holding element n - 1 also writes the total
-    if (threadIdx.x == 0 && start + kScanChunk >= n) out[n] = static_cast<int>(base + total);
+    if (threadIdx.x == 0 && start + kScanChunk >= n) out[n] = scan_offset(base + static_cast<uint32_t>(total));
 }
 
 // ---------------------------------------------------------------- records

@@ -235,7 +235,7 @@ bool MultiViewRenderer::Render(const GaussianBuffers& g, const std::vector<Camer
     // stream waits for all of them
     last_records_ = 0;
     for (size_t k = 0; k < count; ++k) {
-        if (host_totals_[k] < 0) return false;
+        if (host_totals_[k] < 0 || host_totals_[k] == INT_MAX) return false;  // more than an int counts
         views_[k]->records = host_totals_[k];
         last_records_ += host_totals_[k];
         if (!Order(*views_[k], n, side_of(k))) return false;

@@ -222,7 +222,7 @@ bool Renderer::OrderBySort(const uint32_t* by_depth, const int* visible, int cou
                 cudaStreamSynchronize(s) != cudaSuccess)
                 return false;
             records = *host_records_;
-            if (records < 0) return false;
+            if (records < 0 || records == INT_MAX) return false;  // more than an int counts (the scan's limit)
             if (!ReserveAtAnyRate([&] { return ReserveRecords(records) && ReserveSort(records); })) return false;
             last_records_ = records;
         }

@@ -54,3 +54,27 @@ def test_lists_at_the_edges_of_the_sorts_forms(n, capacity, away, fast):
         assert len(ids) < capacity
     got_ids, got_offsets = gsn_sorted_lists(r, cam)
     assert np.array_equal(got_offsets, offsets) and np.array_equal(got_ids, ids)
+
+
+@pytest.mark.parametrize("n", [250_000, 470_000])
+def test_more_records_than_an_int_counts_are_refused_or_reported(n):
+    """Every Gaussian covers all 10,000 tiles: 2.5 and 4.7 billion records, beyond 2^31 and
+    2^32. Grow mode refuses the frame; with a fixed capacity the records that fit are
+    rendered and the overflow flag is set."""
+    t = torch()
+    params = scenes.random_gaussians(n, 4, mean_sigma=0.1)
+    params[2] += 3.0
+    params[3:6] = 4.0
+    cam = scenes.make_camera(1600, 1600, fx=400.0, fy=400.0)
+    p = dev(params)
+    image = empty((1600, 1600, 3), t.float32)
+    assert gsn.Renderer().render(p.data_ptr(), n, cam, [0, 0, 0], image.data_ptr(), 0) != 0
+    r = gsn.Renderer()
+    assert r.set_record_capacity(300_000) == 0
+    assert r.render(p.data_ptr(), n, cam, [0, 0, 0], image.data_ptr(), 0) == 0
+    sync()
+    b = r.buffers()
+    assert host(b.tile_counts, np.int32, n).astype(np.int64).sum() == n * cam.tiles
+    assert host(b.overflow, np.int32, 1)[0] == 1 and bool(t.isfinite(image).all())
+    ids, offsets = gsn_sorted_lists(r, cam)
+    assert offsets[-1] == 300_000 and len(np.unique(ids)) == 30

@@ -142,6 +142,14 @@ def test_exclusive_scan_matches_cumulative_sum(n):
     assert np.array_equal(run_scan(values, in_place=True), expected_scan(values))
 
 
+def test_exclusive_scan_stays_at_the_largest_int():
+    values = np.full(9001, 1_000_003, dtype=np.int32)  # passes 2^31 and 2^32
+    expected = np.minimum(expected_scan(values), 2 ** 31 - 1)
+    assert np.array_equal(run_scan(values), expected)
+    assert np.array_equal(run_scan(values, np.arange(9001)[::-1].copy(), 8000),
+                          np.minimum(expected_scan(values, np.arange(9001), 8000), 2 ** 31 - 1))
+
+
 def test_exclusive_scan_edge_cases():
     t = torch()
     out = dev(np.array([7], dtype=np.int32))
