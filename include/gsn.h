@@ -114,8 +114,8 @@ int gsn_sort_pairs_noalloc(uint32_t* keys, uint32_t* values, uint32_t* keys_alt,
  * the entries before i, out[count] = the total, where entry j is
  * in[gather ? gather[j] : j] for j < *valid (device int; all `count` when
  * valid is null) and zero from there on. `out` holds count + 1 ints; in == out
- * is allowed without `gather`. One pass with decoupled look-back. Device
- * workspace: gsn_exclusive_scan_workspace bytes. */
+ * is allowed without `gather`. Sums beyond INT_MAX stay at INT_MAX. One pass with
+ * decoupled look-back. Device workspace: gsn_exclusive_scan_workspace bytes. */
 int gsn_exclusive_scan_workspace(int max_count, size_t* bytes);
 int gsn_exclusive_scan(const int* in, const uint32_t* gather, int* out, int count, const int* valid,
                        void* workspace, size_t workspace_bytes, void* stream);
